@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "tp_ccg.cuh"
 #include "tp_ops.cuh"
 
 namespace tp {
@@ -782,6 +783,7 @@ struct tp_cg_handle {
   tp::Glob* glob;
   tp::Lanes lanes;
   int32_t* sys_active;
+  tp::Ccg* ccg = nullptr;  // cluster engine (tp_ccg.cu) in place of the graph
 };
 
 namespace tp {
@@ -1124,6 +1126,20 @@ extern "C" int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const 
     delete h;
     return TP_ERR_CUDA;
   }
+  // systems that fit one thread-block cluster each run there; the host-loop variant
+  // (use_graph_loop = 0) always is the graph engine
+  if (h->use_cond) {
+    rc = ccg_create(op, cfg->inner_fp32, CcgSource{}, cfg->max_it, delta, b, x, rtol, st,
+                    &h->ccg);
+    if (rc) {
+      tp_cg_destroy(h);
+      return rc;
+    }
+    if (h->ccg) {
+      *out = h;
+      return TP_OK;
+    }
+  }
   void* arg = h->vt_fp32 ? (void*)&h->af : (void*)&h->ad;
   rc = build_graphs(h, K, arg);
   if (rc) {
@@ -1134,9 +1150,16 @@ extern "C" int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const 
   return TP_OK;
 }
 
+extern "C" int tp_cg_engine(tp_cg_handle* h, int* cluster) {
+  TP_REQUIRE(h && cluster, "null pointer");
+  *cluster = h->ccg ? 1 : 0;
+  return TP_OK;
+}
+
 extern "C" int tp_cg_run(tp_cg_handle* h, void* stream) {
   TP_REQUIRE(h, "null handle");
   cudaStream_t st = as_stream(stream);
+  if (h->ccg) return ccg_run(h->ccg, st);
   if (h->use_cond) {
     TP_CUDA_TRY(cudaGraphLaunch(h->exec, st));
     return TP_OK;
@@ -1160,6 +1183,8 @@ extern "C" int tp_cg_result_get(tp_cg_handle* h, tp_cg_result* res, int32_t* lan
                                 void* stream) {
   TP_REQUIRE(h, "null handle");
   cudaStream_t st = as_stream(stream);
+  if (h->ccg)
+    return ccg_result(h->ccg, res, lane_iters, lane_status, lane_rnorm, lane_bnorm, st);
   Glob g;
   const int NL = h->NL;
   std::vector<int32_t> it(NL), stt(NL);
@@ -1194,6 +1219,7 @@ extern "C" int tp_cg_result_get(tp_cg_handle* h, tp_cg_result* res, int32_t* lan
 
 extern "C" int tp_cg_destroy(tp_cg_handle* h) {
   if (!h) return TP_OK;
+  if (h->ccg) ccg_destroy(h->ccg);
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->e_init) cudaGraphExecDestroy(h->e_init);

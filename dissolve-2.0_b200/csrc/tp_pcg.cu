@@ -48,6 +48,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tp_ccg.cuh"
 #include "tp_ops.cuh"
 
 namespace tp {
@@ -3316,7 +3317,16 @@ struct tp_pcg_handle {
   uint16_t* d_loc_col = nullptr;
   // pipelined engine: bulk-copy runs and single entries of the halo
   void* d_runs = nullptr;
+  // cluster engine (tp_ccg.cu), used in place of the grid engine unless a run is profiled;
+  // the grid engine's window tables are then built late
+  tp::Ccg* ccg = nullptr;
+  bool grid_ready = false, hasM = false, ran_cluster = false;
+  tp_sell sell;
+  bool use_cluster() const {
+    return ccg && !(fp32 ? af.prof : ad.prof);
+  }
   ~tp_pcg_handle() {
+    if (ccg) tp::ccg_destroy(ccg);
     if (d_halo_ptr) cudaFree(d_halo_ptr);
     if (d_halo) cudaFree(d_halo);
     if (d_loc_col) cudaFree(d_loc_col);
@@ -3722,6 +3732,23 @@ static int try_window(tp_pcg_handle* h, const tp_sell* sell, bool hasM, cudaStre
   return TP_OK;
 }
 
+// A system that fits one thread-block cluster runs there, unless the environment names one
+// of the grid engines.
+static bool cluster_allowed() {
+  for (const char* v : {"DISSOLVE_PCG_ENGINE", "DISSOLVE_PCG_PIPE", "DISSOLVE_PCG_CGT",
+                        "DISSOLVE_PCG_TMEM"})
+    if (getenv(v)) return false;
+  return true;
+}
+
+// The grid engine of a handle that runs the cluster engine: its window tables, built when
+// a profile first asks for it.
+static int ready_grid(tp_pcg_handle* h) {
+  if (h->grid_ready) return TP_OK;
+  h->grid_ready = true;
+  return try_window(h, &h->sell, h->hasM, nullptr);
+}
+
 extern "C" int tp_pcg_create(const tp_csr_op* op, const tp_sell* sell, int max_it,
                              int inner_fp32, double delta, int ctas_per_sm, const double* b,
                              double* x, const double* rtol, void* workspace,
@@ -3764,7 +3791,18 @@ extern "C" int tp_pcg_create(const tp_csr_op* op, const tp_sell* sell, int max_i
   h->bar = h->fp32 ? h->af.bar : h->ad.bar;
   h->out = h->fp32 ? h->af.out : h->ad.out;
   cudaStream_t st = as_stream(stream);
-  rc = try_window(h, sell, hasM, st);
+  h->sell = *sell;
+  h->hasM = hasM;
+  if (cluster_allowed() && !hasM && ctas_per_sm <= 0) {
+    CcgSource src;
+    src.sK = inner_fp32 ? (const void*)sell->sK32 : (const void*)sell->sK64;
+    src.slice_ptr = sell->slice_ptr;
+    rc = ccg_create(op, h->fp32, src, max_it, d, b, x, rtol, st, &h->ccg);
+  }
+  if (rc == TP_OK && !h->ccg) {
+    rc = try_window(h, sell, hasM, st);
+    h->grid_ready = true;
+  }
   if (rc != TP_OK) {
     delete h;
     return rc;
@@ -3784,6 +3822,8 @@ extern "C" int tp_pcg_create(const tp_csr_op* op, const tp_sell* sell, int max_i
 extern "C" int tp_pcg_run(tp_pcg_handle* h, void* stream) {
   TP_REQUIRE(h, "null handle");
   cudaStream_t st = as_stream(stream);
+  h->ran_cluster = h->use_cluster();
+  if (h->ran_cluster) return ccg_run(h->ccg, st);
   // a previous run that timed out leaves the abort flag set: clear the barrier first
   TP_CUDA_TRY(cudaMemsetAsync(h->bar, 0, sizeof(PBar), st));
   void* arg = h->fp32 ? (void*)&h->af : (void*)&h->ad;
@@ -3798,6 +3838,8 @@ extern "C" int tp_pcg_result_get(tp_pcg_handle* h, tp_cg_result* res, int32_t* l
                                  void* stream) {
   TP_REQUIRE(h, "null handle");
   cudaStream_t st = as_stream(stream);
+  if (h->ran_cluster)
+    return ccg_result(h->ccg, res, lane_iters, lane_status, lane_rnorm, lane_bnorm, st);
   POut o;
   TP_CUDA_TRY(cudaMemcpyAsync(&o, h->out, sizeof(POut), cudaMemcpyDeviceToHost, st));
   TP_CUDA_TRY(cudaStreamSynchronize(st));
@@ -3826,13 +3868,18 @@ extern "C" int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block) {
 
 extern "C" int tp_pcg_engine(tp_pcg_handle* h, int* window, size_t* smem_bytes) {
   TP_REQUIRE(h, "null handle");
-  if (window) *window = h->window;
+  if (window) *window = h->ccg ? 4 : h->window;
   if (smem_bytes) *smem_bytes = h->dyn_smem;
+  if (smem_bytes && h->ccg) *smem_bytes = ccg_smem(h->ccg);
   return TP_OK;
 }
 
 extern "C" int tp_pcg_set_profile(tp_pcg_handle* h, unsigned long long* prof) {
   TP_REQUIRE(h, "null handle");
+  if (prof) {
+    const int rc = ready_grid(h);
+    if (rc != TP_OK) return rc;
+  }
   h->af.prof = prof;
   h->ad.prof = prof;
   return TP_OK;
@@ -3845,6 +3892,7 @@ extern "C" int tp_pcg_set_wait_limit(tp_pcg_handle* h, unsigned long long limit_
   const unsigned long long lim = limit_ns ? limit_ns : WAIT_LIMIT_NS;
   h->af.wait_limit_ns = h->ad.wait_limit_ns = lim;
   h->af.wait_missing = h->ad.wait_missing = missing_arrivals;
+  if (h->ccg) ccg_set_wait(h->ccg, lim, missing_arrivals);
   return TP_OK;
 }
 

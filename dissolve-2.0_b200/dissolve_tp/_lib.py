@@ -155,6 +155,7 @@ SIGNATURES = {
     "tp_cg_workspace_bytes": (ctypes.c_size_t, [_P(TpCsrOp), _P(TpCgConfig)]),
     "tp_cg_create": (ctypes.c_int, [_P(TpCsrOp), _P(TpCgConfig), _vp, _vp, _vp, _vp,
                                     ctypes.c_size_t, _vp, _P(_vp)]),
+    "tp_cg_engine": (ctypes.c_int, [_vp, _P(ctypes.c_int)]),
     "tp_cg_run": (ctypes.c_int, [_vp, _vp]),
     "tp_cg_result_get": (ctypes.c_int, [_vp, _P(TpCgResult), _vp, _vp, _vp, _vp, _vp]),
     "tp_cg_destroy": (ctypes.c_int, [_vp]),

@@ -78,13 +78,18 @@ class MeshBatch:
         self.op = CsrOperator(dm.indptr, dm.indices[: dm.nnz], self.K64, K32=self.K32,
                               n_systems=self.n_meshes, sys_row_ptr=vp)
         cg = dict(cg or {})
-        if autotune and not {"group", "block", "rows_per_tile"} & set(cg):
-            self.assemble_operator()
-            cg.update(tune_cg(self.op, inner_fp32=inner_fp32))
-        self.cg_config = dict(cg, engine="graph", n_systems=self.n_meshes)
+        self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32, **cg)
+        if self.solver.cluster():
+            self.cg_config = dict(engine="cluster", n_systems=self.n_meshes)
+        else:
+            if autotune and not {"group", "block", "rows_per_tile"} & set(cg):
+                self.assemble_operator()
+                cg.update(tune_cg(self.op, inner_fp32=inner_fp32))
+                self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32,
+                                       **cg)
+            self.cg_config = dict(cg, engine="graph", n_systems=self.n_meshes)
         if asm_tiles is not None:
             self.cg_config["assembly_rows_per_tile"] = asm_tiles
-        self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32, **cg)
         self.U = torch.zeros(dm.n_verts, dtype=torch.float64, device=dev)
 
     @property

@@ -105,6 +105,13 @@ class CGSolver:
         r = np.broadcast_to(np.asarray(rtol, dtype=np.float64), (self.n_lanes,))
         self.rtol.copy_(torch.from_numpy(np.array(r, dtype=np.float64)))
 
+    def cluster(self) -> bool:
+        """Whether every system is solved by one thread-block cluster (the launch shape
+        group/block/rows_per_tile then has no effect)."""
+        c = ctypes.c_int(0)
+        call("tp_cg_engine", self._h, ctypes.byref(c))
+        return bool(c.value)
+
     def run(self):
         """Enqueue one solve on the current stream (no host synchronisation)."""
         call("tp_cg_run", self._h, stream_handle())
@@ -257,11 +264,11 @@ class PersistentCG:
     def engine(self) -> dict:
         """Engine of the handle: shared-memory window (Chronopoulos-Gear; `tmem`: with the
         recurrence vectors in tensor memory; `pipelined`: the one-barrier pipelined form,
-        vectors in tensor memory) or streaming."""
+        vectors in tensor memory; `cluster`: one thread-block cluster) or streaming."""
         w, sm = ctypes.c_int(0), ctypes.c_size_t(0)
         call("tp_pcg_engine", self._h, ctypes.byref(w), ctypes.byref(sm))
-        return {"window": bool(w.value), "tmem": w.value >= 2, "pipelined": w.value == 3,
-                "smem_bytes": int(sm.value)}
+        return {"window": bool(w.value), "tmem": w.value in (2, 3), "pipelined": w.value == 3,
+                "cluster": w.value == 4, "smem_bytes": int(sm.value)}
 
     def run(self):
         call("tp_pcg_run", self._h, stream_handle())

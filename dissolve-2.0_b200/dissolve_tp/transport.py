@@ -161,6 +161,7 @@ class BatchedTransport:
             self.cg_config["grid"], self.cg_config["block"] = self.solver.grid()
             eng = self.solver.engine()
             self.cg_config["form"] = (
+                "cluster (Chronopoulos-Gear, one thread-block cluster)" if eng["cluster"] else
                 "window (pipelined, vectors in tensor memory)" if eng["pipelined"] else
                 "window (Chronopoulos-Gear, vectors in tensor memory)" if eng["tmem"] else
                 "window (Chronopoulos-Gear)" if eng["window"] else "streaming")

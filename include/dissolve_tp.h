@@ -447,6 +447,12 @@ TP_API int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const doub
                  const double* rtol, void* workspace, size_t workspace_bytes, void* stream,
                  tp_cg_handle** out);
 
+/* Engine the handle runs (chosen at create).  *cluster = 1: every system is solved by one
+ * thread-block cluster (all systems fit one: about 70k rows for one FP32 column, 49k for
+ * one FP64 column, 24k for 4 FP32 columns; no mass matrix; use_graph_loop = 1), which
+ * ignores group, block and rows_per_tile; 0: the graph engine. */
+TP_API int tp_cg_engine(tp_cg_handle* h, int* cluster);
+
 /* enqueue one solve (recomputes the Jacobi diagonal from the current values) */
 TP_API int tp_cg_run(tp_cg_handle* h, void* stream);
 
@@ -509,6 +515,7 @@ TP_API int tp_pcg_run(tp_pcg_handle* h, void* stream);
 TP_API int tp_pcg_result_get(tp_pcg_handle* h, tp_cg_result* res, int32_t* lane_iters,
                              int32_t* lane_status, double* lane_rnorm, double* lane_bnorm,
                              void* stream);
+/* grid and block of the handle's grid engine (the shape a profile array is sized by) */
 TP_API int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block);
 /* Engine the handle runs (chosen at create).  *window = 1: the window engine -- the
  * Chronopoulos-Gear form of the same Jacobi-PCG, in which the only vector shared between
@@ -523,7 +530,11 @@ TP_API int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block);
  * one grid barrier per iteration; its FP64 refreshes restart the refreshed lanes) with
  * the same tensor-memory layout, for at most 3 columns (DISSOLVE_PCG_PIPE=0 at create keeps
  * engine 2); it refreshes at least every factor 1e3 of residual reduction whatever
- * `delta` asks for.  *window = 0: the streaming engine (standard recurrences, columns and
+ * `delta` asks for.  *window = 4: the Chronopoulos-Gear form in one thread-block cluster,
+ * for a system that fits one (as for tp_cg_engine; not when the environment names one of
+ * the grid engines through a DISSOLVE_PCG_* variable, or ctas_per_sm is given); profiled
+ * runs use the grid engine of the handle.
+ * *window = 0: the streaming engine (standard recurrences, columns and
  * gathers from global memory).  *smem_bytes: dynamic shared memory per CTA.  The
  * environment variable DISSOLVE_PCG_ENGINE=stream at create forces the streaming
  * engine. */
