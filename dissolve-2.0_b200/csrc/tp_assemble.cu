@@ -406,15 +406,16 @@ __global__ void __launch_bounds__(TILE_BLOCK, 3) k_assemble_tiles(
       for (int g = 3; more && 8 * g < KD; g++) more = group(__ldg(dv + g));
     }
     const double v = is_bc ? 1.0 : dacc;
-    if (out64) out64[pd] = v;
-    if (out32) out32[pd] = (float)v;
+    // a vertex no cell uses has an empty row (pd = -1)
+    if (out64 && pd >= 0) out64[pd] = v;
+    if (out32 && pd >= 0) out32[pd] = (float)v;
     if (ex.sell32) {
       // the diagonal, then the row's padding entries of its SELL-32 slice
       const int p0 = __ldg(indptr + r), len = __ldg(indptr + r + 1) - p0;
       const int64_t sl = r >> 5;
       const int base = ex.slice_ptr[sl], width = (ex.slice_ptr[sl + 1] - base) >> 5;
       float* col = ex.sell32 + base + (r & 31);
-      col[(int64_t)(pd - p0) * 32] = (float)v;
+      if (pd >= 0) col[(int64_t)(pd - p0) * 32] = (float)v;
       for (int k = len; k < width; k++) col[(int64_t)k * 32] = 0.f;
     }
     if constexpr (DIAG) {

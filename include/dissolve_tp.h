@@ -126,11 +126,10 @@ TP_API int tp_incidence_slots(const tp_mesh* m, uint32_t* slots, int32_t* flags_
 
 /* [sync] Row tiles for the tiled kernels (no reference counterpart): the rows are cut by
  * recursive coordinate bisection into tiles of rows_per_tile (64) nearby rows; per tile
- * the ascending list of the distinct cells its rows touch and, per incidence entry of its
- * rows (row-major [entry k][row]), the cell's tile-local index, the row's local vertex
- * and the four CSR slots of tp_incidence_slots.  Needs a complete mesh (coords4, v2c,
- * v2c_slots, indptr); built on the host from copies of those arrays, device tables owned
- * by the returned handle.  TP_ERR_CAPACITY if a tile touches more than 16383 cells. */
+ * the ascending list of the distinct cells its rows touch and, per row and per owned
+ * edge, its cells as positions in that list.  Needs a complete mesh (coords4, v2c,
+ * v2c_slots, indptr); built on the GPU, device tables owned by the returned handle.
+ * TP_ERR_CAPACITY if a tile touches more than 4095 cells. */
 TP_API int tp_tiles_create(const tp_mesh* m, int rows_per_tile, void* stream, tp_tiles** out);
 /* size of the tiling (any pointer may be NULL) */
 TP_API int tp_tiles_info(const tp_tiles* t, int32_t* n_tiles, int32_t* rows_per_tile,
