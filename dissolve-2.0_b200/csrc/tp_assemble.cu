@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128) k_assemble_rows(
         const GeoRec& g = gv[u];
         if constexpr (DIAG) {
           const int64_t c = ev[u] >> 2;
-          const double Ld = __dmul_rn(__ddiv_rn(g.dJ, 120.0), 5.0);
+          const double Ld = __dmul_rn(div120(g.dJ), 5.0);
 #pragma unroll
           for (int s = 0; s < 4; s++) {
             if (s < ex.S) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128) k_assemble_rows(
         double kr[4];
         kref_row(li, g, kr);
         const double kscale = (MODE == TP_ASM_MASS) ? 0.0
-                                                    : __ddiv_rn(__dmul_rn(g.dJ, dev[u]), 6.0);
+                                                    : div6(__dmul_rn(g.dJ, dev[u]));
         const double react = (MODE == TP_ASM_FULL) ? __dadd_rn(inv_dt, alv[u]) : 1.0;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -223,7 +223,7 @@ __device__ __forceinline__ void tile_cell_entries(double* slot, bool has_alpha, 
   const GeoRec g{r[0], r[1], r[2], r[3], r[4], r[5], r[6]};
   const double de = (MODE == TP_ASM_MASS) ? 0.0 : r[8];
   const double al = (MODE == TP_ASM_FULL && has_alpha) ? r[9] : 0.0;
-  const double ks = (MODE == TP_ASM_MASS) ? 0.0 : __ddiv_rn(__dmul_rn(g.dJ, de), 6.0);
+  const double ks = (MODE == TP_ASM_MASS) ? 0.0 : div6(__dmul_rn(g.dJ, de));
   const double react = (MODE == TP_ASM_FULL) ? __dadd_rn(inv_dt, al) : 1.0;
   double e[10];
 #pragma unroll
@@ -242,9 +242,9 @@ __device__ __forceinline__ void tile_cell_entries(double* slot, bool has_alpha, 
     for (int k = 0; k < 5; k++) sts2(slot + 2 * k, e[2 * k], e[2 * k + 1]);
   }
   if constexpr (DIAG && CMP) {
-    slot[10] = __dmul_rn(__ddiv_rn(g.dJ, 120.0), 5.0);
+    slot[10] = __dmul_rn(div120(g.dJ), 5.0);
   } else if constexpr (DIAG) {
-    const double Ld = __dmul_rn(__ddiv_rn(g.dJ, 120.0), 5.0);
+    const double Ld = __dmul_rn(div120(g.dJ), 5.0);
     double dt[4];
 #pragma unroll
     for (int s = 0; s < 4; s++)
@@ -511,7 +511,7 @@ __global__ void k_cell_average(int64_t n, const int4* __restrict__ cells,
        c += (int64_t)gridDim.x * blockDim.x) {
     const int4 v = cells[c];
     const double s = __dadd_rn(__dadd_rn(__dadd_rn(vv[v.x], vv[v.y]), vv[v.z]), vv[v.w]);
-    out[c] = __ddiv_rn(s, 4.0);
+    out[c] = __dmul_rn(s, 0.25);
   }
 }
 
@@ -540,7 +540,7 @@ __global__ void k_lumped_diag(int64_t nv, int S, int ld, const int32_t* __restri
 #pragma unroll
         for (int u = 0; u < PF; u++) {
           if (k0 + u >= kend) break;
-          const double Ld = __dmul_rn(__ddiv_rn(dJ[u], 120.0), 5.0);
+          const double Ld = __dmul_rn(div120(dJ[u]), 5.0);
 #pragma unroll
           for (int s = 0; s < 4; s++) {
             if (s < S) {
@@ -591,7 +591,7 @@ __global__ void k_rhs_rows(int64_t nv, int S, int ld, const int32_t* __restrict_
       for (int q = 0; q < PF; q++) {
         if (k0 + q >= kend) break;
         const int64_t c = cvv[q];
-        const double base = __ddiv_rn(dJv[q], 120.0);
+        const double base = div120(dJv[q]);
         if (lumped) {
           const double Ld = __dmul_rn(base, 5.0);
 #pragma unroll
@@ -630,9 +630,14 @@ __global__ void k_rhs_rows(int64_t nv, int S, int ld, const int32_t* __restrict_
 // Right-hand side on row tiles: the tile's cells' factors in shared memory, then each
 // tile row sums its cells in ascending order -- the same ordered sums, with the same
 // rounding, as k_rhs_rows.  Lumped: one slot per cell, Ld = (|detJ| / 120) 5, and the row
-// adds Ld (inv_dt u + f).  Consistent: a slot of CW = 6 (10 with f) doubles per cell,
-// [base dt^-1, base, sum of u over the cell's vertices (4 columns), the same for f], base =
-// |detJ| / 120, and the row adds base dt^-1 (su + u_r) + base (sf + f_r).
+// adds Ld (inv_dt u + f).  Consistent: a slot of CW doubles per cell, [base dt^-1, base, sum
+// of u over the cell's vertices (S columns), the same for f], base = |detJ| / 120, and the
+// row adds base dt^-1 (su + u_r) + base (sf + f_r).  CW is odd (consecutive slots in
+// different banks) and no wider than S needs: it sets how many tiles share an SM.
+__host__ __device__ inline int rhs_slot_width(bool lumped, int S, bool f) {
+  return lumped ? 1 : (2 + (f ? 2 : 1) * S) | 1;
+}
+
 template <bool LUMPED>
 __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
                                                    const int32_t* __restrict__ cells,
@@ -643,7 +648,7 @@ __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
   extern __shared__ double sm_ld[];
   const int R = tv.R, T = blockDim.x, t = blockIdx.x, tid = threadIdx.x;
   const int c0 = __ldg(tv.cell_ptr + t), m = __ldg(tv.cell_ptr + t + 1) - c0;
-  const int CW = LUMPED ? 1 : (f ? 10 : 6);
+  const int CW = rhs_slot_width(LUMPED, S, f != nullptr), FO = 2 + S;
   {
     constexpr int MAXC = 4;
     int64_t cid[MAXC];
@@ -664,9 +669,9 @@ __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
     auto put = [&](int i, double djv, const int4& c4) {
       double* slot = sm_ld + (size_t)i * CW;
       if constexpr (LUMPED) {
-        slot[0] = __dmul_rn(__ddiv_rn(djv, 120.0), 5.0);
+        slot[0] = __dmul_rn(div120(djv), 5.0);
       } else {
-        const double base = __ddiv_rn(djv, 120.0);
+        const double base = div120(djv);
         slot[0] = __dmul_rn(base, inv_dt);
         slot[1] = base;
 #pragma unroll
@@ -677,7 +682,7 @@ __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
                         __ldg(u + (int64_t)c4.z * ld + s)),
               __ldg(u + (int64_t)c4.w * ld + s));
           if (f)
-            slot[6 + s] = __dadd_rn(
+            slot[FO + s] = __dadd_rn(
                 __dadd_rn(__dadd_rn(__ldg(f + (int64_t)c4.x * ld + s), __ldg(f + (int64_t)c4.y * ld + s)),
                           __ldg(f + (int64_t)c4.z * ld + s)),
                 __ldg(f + (int64_t)c4.w * ld + s));
@@ -741,7 +746,7 @@ __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
 #pragma unroll
         for (int s = 0; s < 4; s++) {
           if (s >= S) continue;
-          const double sf = f ? slot[6 + s] : 0.0;
+          const double sf = f ? slot[FO + s] : 0.0;
           acc[s] = __dadd_rn(acc[s], __dadd_rn(__dmul_rn(mdt, __dadd_rn(slot[2 + s], w[s])),
                                                __dmul_rn(base, __dadd_rn(sf, fr[s]))));
         }
@@ -831,7 +836,7 @@ __global__ void k_nodal_gradient(int64_t nv, const int32_t* __restrict__ cells,
                                   __dmul_rn(JT[5], g2));
       const double pz = __dadd_rn(__dadd_rn(__dmul_rn(JT[6], g0), __dmul_rn(JT[7], g1)),
                                   __dmul_rn(JT[8], g2));
-      const double w = __ddiv_rn(geo[8 * c + 6], 6.0);
+      const double w = div6(geo[8 * c + 6]);
       gx = __dadd_rn(gx, __dmul_rn(w, px));
       gy = __dadd_rn(gy, __dmul_rn(w, py));
       gz = __dadd_rn(gz, __dmul_rn(w, pz));
@@ -950,7 +955,7 @@ __global__ void k_cell_average_col(int64_t n, const int4* __restrict__ cells,
        c += (int64_t)gridDim.x * blockDim.x) {
     const int4 v = cells[c];
     const double s = __dadd_rn(__dadd_rn(__dadd_rn(vv[v.x], vv[v.y]), vv[v.z]), vv[v.w]);
-    out[c * ld + col] = __ddiv_rn(s, 4.0);
+    out[c * ld + col] = __dmul_rn(s, 0.25);
   }
 }
 
@@ -1338,7 +1343,7 @@ extern "C" int tp_assemble_rhs(const tp_mesh* m, int S, int ld, const double* u_
     TP_CUDA_TRY(cudaGetDevice(&dev));
     TP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   }
-  const size_t cw = lumped ? 1 : (f ? 10 : 6);  // k_rhs_tiles' slot width
+  const size_t cw = (size_t)rhs_slot_width(lumped != 0, S, f != nullptr);
   const size_t smem_t = m->tiles ? sizeof(double) * cw * (size_t)std::max(m->tiles->v.max_cells, 1) : 0;
   if (m->n_verts > 0 && m->tiles && m->tiles->v.n_tiles > 0 && m->tiles->v.R <= 256 &&
       smem_t <= (size_t)optin) {

@@ -2,12 +2,26 @@
 //
 // The element entries follow the reference kernel's operation order
 // (gpu/gpu_assembler.py:104-132) with every product and sum rounded separately
-// (__dmul_rn/__dadd_rn/__ddiv_rn: no FMA contraction), so that a row summed over its
+// (__dmul_rn/__dadd_rn, div6/div120: no FMA contraction), so that a row summed over its
 // cells in ascending cell order equals the reference kernel executed in cell order.
 #pragma once
 #include "tp_common.cuh"
 
 namespace tp {
+
+// x / 6 and x / 120 rounded to nearest, in two operations: the division by a constant of
+// Brisebarre, Muller and Raina (IEEE Trans. Computers 53(8), 2004), x c_h + RN(x c_l) with
+// c_h = RN(1/c), c_l = RN(1/c - c_h).  For c = 6 and 120 it is the correctly rounded quotient
+// for every x: the divisor's odd part (3, 15) keeps x / c at least 1/30 of a unit in the
+// last place from every rounding boundary, and the fused sum is within 2^-50 of a unit.
+// (Below 1e-290 x c_l underflows and the last bit may differ.)  A division here costs about
+// ten times as many instructions, and the element kernels do two per cell.
+__device__ __forceinline__ double div6(double x) {
+  return __fma_rn(x, 0x1.5555555555555p-3, __dmul_rn(x, 0x1.5555555555555p-57));
+}
+__device__ __forceinline__ double div120(double x) {
+  return __fma_rn(x, 0x1.1111111111111p-7, __dmul_rn(x, 0x1.1111111111111p-63));
+}
 
 struct GeoRec {
   double G00, G01, G02, G11, G12, G22, dJ;
@@ -55,9 +69,9 @@ __device__ __forceinline__ double elem_entry(const double kr[4], int i, int j, d
   if (MODE != TP_ASM_STIFF) {
     double M;
     if (lumped)
-      M = (i == j) ? __ddiv_rn(__dmul_rn(dJ, 5.0), 120.0) : 0.0;
+      M = (i == j) ? div120(__dmul_rn(dJ, 5.0)) : 0.0;
     else
-      M = __ddiv_rn(__dmul_rn(dJ, (i == j) ? 2.0 : 1.0), 120.0);
+      M = div120(__dmul_rn(dJ, (i == j) ? 2.0 : 1.0));
     a = (MODE == TP_ASM_FULL) ? __dadd_rn(a, __dmul_rn(react, M)) : M;
   }
   return a;
