@@ -171,20 +171,25 @@ __global__ void __launch_bounds__(128) k_assemble_rows(
 // ----------------------------------------------------------------- tiled CSR assembly
 // One CTA per row tile (tp_tiles.cu).  Phase A: the records of the tile's distinct cells
 // are copied into shared memory with asynchronous copies, all in flight together; each
-// cell's 10 upper-triangle entries (elem_entry, the reference's rounding) and, with DIAG,
-// its S lumped-diagonal terms replace its record in place (odd slot stride: the cells the
-// lanes of a warp read fall in different banks).  Phase B: each
+// cell's 10 upper-triangle entries (elem_entry, the reference's rounding) replace its record
+// in place, and with DIAG its lumped-diagonal terms go to a second array.  Phase B: each
 // tile row sums its diagonal over its cells in ascending order, each owned edge sums its
 // cells in ascending order, in registers, and writes (r, v) and (v, r) -- the same
 // ordered sums as the row walk of k_assemble_rows, bit for bit.
+//
+// What bounds it: latency within a tile (three CTAs of the largest tiles per SM; more
+// threads per CTA, 32-row tiles, record loads straight into registers and L2 prefetches of
+// later tiles all measured slower).  So a tile's loads hang on one header load, and the
+// sums of phase B run without branches, their shared-memory reads in flight together.
 constexpr int TILE_BLOCK = 256;
 
-// Shared-memory slot of one cell: ew doubles, ew = 10 or 14 (80 or 112 bytes: 5 or 7
-// sixteen-byte units, so 16-byte accesses of 8 consecutive slots fall in 8 different
-// bank groups).  First the raw record as copied -- the 64-byte geometry record
-// (G00 G01 G02 G11 G12 G22 |detJ| 0) at 0..7, De at 8, alpha at 9 or the DIAG alpha
-// columns at 9..9+ld-1 -- then, computed in place by one thread, the 10 upper-triangle
-// entries at 0..9 and, with DIAG, the S lumped-diagonal column terms at 10..10+S-1.
+// Shared-memory slot of one cell: 10 doubles (80 bytes, 5 sixteen-byte units, so 16-byte
+// accesses of 8 consecutive slots fall in 8 different bank groups).  First the raw record
+// as copied -- the 64-byte geometry record (G00 G01 G02 G11 G12 G22 |detJ| 0) at 0..7, De
+// at 8, alpha at 9 -- then, computed in place by one thread, the 10 upper-triangle entries.
+// Slot m (past the tile's cells) holds zeros: the padding terms read it.
+constexpr int TILE_EW = 10;
+
 __device__ __forceinline__ void lds2(const double* p, double& a, double& b) {
   const double2 v = *reinterpret_cast<const double2*>(p);
   a = v.x;
@@ -194,32 +199,17 @@ __device__ __forceinline__ void sts2(double* p, double a, double b) {
   *reinterpret_cast<double2*>(p) = make_double2(a, b);
 }
 
-// CMP (compact, DIAG without per-cell alpha): ew = 11, the slot keeps only the cell's
-// lumped-mass factor Ld at 10 (each column's term shift_s Ld is formed where it is summed,
-// with the same rounding); the odd stride leaves slots 8-byte aligned only, so every
-// access is a single double.
+// DIAG keeps nd doubles per cell beside the slots: without per-cell alpha (CMP) the cell's
+// lumped-mass factor Ld alone (each column's term shift_s Ld is formed where it is summed,
+// with the same rounding), with it the S column terms (first the raw alpha columns).
 template <int MODE, bool DIAG, bool CMP = false>
-__device__ __forceinline__ void tile_cell_entries(double* slot, bool has_alpha, double inv_dt,
-                                                  int lumped, const RowExtras& ex,
+__device__ __forceinline__ void tile_cell_entries(double* slot, double* xd, bool has_alpha,
+                                                  double inv_dt, int lumped, const RowExtras& ex,
                                                   const double dsh[4]) {
   // the whole raw record first (the entries overwrite it)
   double r[10];
-  if constexpr (CMP) {
 #pragma unroll
-    for (int k = 0; k < 10; k++) r[k] = slot[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 5; k++) lds2(slot + 2 * k, r[2 * k], r[2 * k + 1]);
-  }
-  double alc[4] = {0.0, 0.0, 0.0, 0.0};
-  if constexpr (DIAG && !CMP) {
-    if (ex.alpha) {
-      alc[0] = r[9];
-#pragma unroll
-      for (int s = 1; s < 4; s++)
-        if (s < ex.ld) alc[s] = slot[9 + s];
-    }
-  }
+  for (int k = 0; k < 5; k++) lds2(slot + 2 * k, r[2 * k], r[2 * k + 1]);
   const GeoRec g{r[0], r[1], r[2], r[3], r[4], r[5], r[6]};
   const double de = (MODE == TP_ASM_MASS) ? 0.0 : r[8];
   const double al = (MODE == TP_ASM_FULL && has_alpha) ? r[9] : 0.0;
@@ -234,23 +224,17 @@ __device__ __forceinline__ void tile_cell_entries(double* slot, bool has_alpha, 
     for (int j = li; j < 4; j++)
       e[tri_index(li, j)] = elem_entry<MODE>(kr, li, j, g.dJ, ks, react, lumped);
   }
-  if constexpr (CMP) {
 #pragma unroll
-    for (int k = 0; k < 10; k++) slot[k] = e[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 5; k++) sts2(slot + 2 * k, e[2 * k], e[2 * k + 1]);
-  }
-  if constexpr (DIAG && CMP) {
-    slot[10] = __dmul_rn(div120(g.dJ), 5.0);
-  } else if constexpr (DIAG) {
+  for (int k = 0; k < 5; k++) sts2(slot + 2 * k, e[2 * k], e[2 * k + 1]);
+  if constexpr (DIAG) {
     const double Ld = __dmul_rn(div120(g.dJ), 5.0);
-    double dt[4];
+    if constexpr (CMP) {
+      xd[0] = Ld;
+    } else {
 #pragma unroll
-    for (int s = 0; s < 4; s++)
-      dt[s] = (s < ex.S) ? __dmul_rn(__dadd_rn(dsh[s], alc[s]), Ld) : 0.0;
-    sts2(slot + 10, dt[0], dt[1]);
-    sts2(slot + 12, dt[2], dt[3]);
+      for (int s = 0; s < 4; s++)
+        if (s < ex.S) xd[s] = __dmul_rn(__dadd_rn(dsh[s], ex.alpha ? xd[s] : 0.0), Ld);
+    }
   }
 }
 
@@ -265,115 +249,118 @@ __device__ __forceinline__ uint32_t term_of(const uint4& v, int k) {
   return (k & 1) ? (w >> 16) : (w & 0xffffu);
 }
 
+// acc + the entries of 8 terms, in order
+__device__ __forceinline__ double add_terms(const double* E, const uint4& g8, double acc) {
+  double v[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const uint32_t tm = term_of(g8, k);
+    v[k] = E[(tm & TILE_LOC_MASK) * TILE_EW + (tm >> TILE_LOC_BITS)];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) acc = __dadd_rn(acc, v[k]);
+  return acc;
+}
+
 template <int MODE, bool DIAG, bool CMP = false>
 __global__ void __launch_bounds__(TILE_BLOCK, 3) k_assemble_tiles(
     TileView tv, const double* __restrict__ geo, const double* __restrict__ De,
     const double* __restrict__ alpha, double inv_dt, int lumped,
     const uint8_t* __restrict__ bc_mask, const int32_t* __restrict__ indptr,
-    double* __restrict__ out64, float* __restrict__ out32, RowExtras ex, int ew, int64_t nv) {
+    double* __restrict__ out64, float* __restrict__ out32, RowExtras ex, int nd, int64_t nv) {
   extern __shared__ double sm_tiles[];
-  const int R = tv.R, T = blockDim.x;
-  const int t = blockIdx.x, tid = threadIdx.x;
-  const int c0 = __ldg(tv.cell_ptr + t), m = __ldg(tv.cell_ptr + t + 1) - c0;
-  double* E = sm_tiles;
+  constexpr int T = TILE_BLOCK;
+  const int R = tv.R, t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  double* const E = sm_tiles;
+  double* const X = E + (size_t)(tv.max_cells + 1) * TILE_EW;  // DIAG: nd doubles per cell
   const double dsh[4] = {ex.shift.x, ex.shift.y, ex.shift.z, ex.shift.w};
-  const uint4 none4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-
-  // ---- phase A: every record of the tile copied into shared memory at once: the ids
-  // first, then the 64-byte geometry records as 16-byte chunks (four lanes per record,
-  // consecutive records on consecutive lanes), De and alpha as 8-byte copies ...
-  {
-    constexpr int MAXC = 4;
-    const int lane = tid & 31;
-    int64_t cid[MAXC];
-#pragma unroll
-    for (int u = 0; u < MAXC; u++) {
-      const int i = tid + u * T;
-      cid[u] = (i < m) ? (int64_t)__ldg(tv.cells + c0 + i) : -1;
-    }
-#pragma unroll
-    for (int u = 0; u < MAXC; u++) {
-      const int ib = (tid & ~31) + u * T;  // the warp's first cell of this round
-      if (ib >= m) break;
-      const int h = lane & 3;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int j = (lane >> 2) + 8 * k;
-        const int64_t c = __shfl_sync(0xffffffffu, cid[u], j);
-        if (ib + j < m) {
-          if constexpr (CMP) {
-            cp_async<8>(E + (size_t)(ib + j) * ew + 2 * h, geo + 8 * c + 2 * h);
-            cp_async<8>(E + (size_t)(ib + j) * ew + 2 * h + 1, geo + 8 * c + 2 * h + 1);
-          } else {
-            cp_async<16>(E + (size_t)(ib + j) * ew + 2 * h, geo + 8 * c + 2 * h);
-          }
-        }
-      }
-      if (cid[u] >= 0) {
-        double* slot = E + (size_t)(ib + lane) * ew;
-        const int64_t c = cid[u];
-        if (MODE != TP_ASM_MASS) cp_async<8>(slot + 8, De + c);
-        if (MODE == TP_ASM_FULL && alpha) cp_async<8>(slot + 9, alpha + c);
-        if constexpr (DIAG && !CMP) {
-          if (ex.alpha)
-            for (int s = 0; s < ex.ld; s++) cp_async<8>(slot + 9 + s, ex.alpha + c * ex.ld + s);
-        }
-      }
-    }
-    for (int i = tid + MAXC * T; i < m; i += T) {  // tiles of more than MAXC * T cells
-      const int64_t c = __ldg(tv.cells + c0 + i);
-      double* slot = E + (size_t)i * ew;
-      if constexpr (CMP) {
-#pragma unroll
-        for (int h = 0; h < 8; h++) cp_async<8>(slot + h, geo + 8 * c + h);
-      } else {
-#pragma unroll
-        for (int h = 0; h < 4; h++) cp_async<16>(slot + 2 * h, geo + 8 * c + 2 * h);
-      }
-      if (MODE != TP_ASM_MASS) cp_async<8>(slot + 8, De + c);
-      if (MODE == TP_ASM_FULL && alpha) cp_async<8>(slot + 9, alpha + c);
-      if constexpr (DIAG && !CMP) {
-        if (ex.alpha)
-          for (int s = 0; s < ex.ld; s++) cp_async<8>(slot + 9 + s, ex.alpha + c * ex.ld + s);
-      }
-    }
-  }
-  // ... while they fly, the phase-B inputs of this thread: its row's first 24 diagonal
-  // terms and its first two edges with their first 8 terms ...
   int64_t r = -1;
-  int pd = 0, KD = 0;
-  const uint4* dv = nullptr;
-  uint4 dq[3] = {none4, none4, none4};
+  int pd = -1;
   if (tid < R) {
     r = __ldg(tv.rows + (int64_t)t * R + tid);
     pd = __ldg(tv.diag_pos + (int64_t)t * R + tid);
-    const int d0 = __ldg(tv.dterm_ptr + t);
-    KD = (__ldg(tv.dterm_ptr + t + 1) - d0) / R;
-    dv = reinterpret_cast<const uint4*>(tv.dterms + d0 + (int64_t)tid * KD);
+  }
+  const TileHead h = tile_head(tv, t);
+  const int m = h.m;
+
+  // ---- phase A: the ids of the cells whose records this warp copies (32 consecutive cells
+  // a round, a record by four lanes as 16-byte chunks) and this thread's own ...
+  constexpr int MAXC = 4;
+  const int32_t* const ids = tv.cells + h.c0;
+  int32_t cq[MAXC][4], cid[MAXC];
+#pragma unroll
+  for (int u = 0; u < MAXC; u++) {
+    const int ib = (tid & ~31) + u * T;  // the warp's first cell of this round
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int j = ib + (lane >> 2) + 8 * k;
+      cq[u][k] = (j < m) ? __ldg(ids + j) : -1;
+    }
+    cid[u] = (ib + lane < m) ? __ldg(ids + ib + lane) : -1;
+  }
+  // ... the phase-B inputs of this thread: its row's first 24 diagonal terms and its first
+  // two edges with their first 8 terms (the diagonal threads take the last edges of a round,
+  // the others the first) ...
+  const uint4* const dv = reinterpret_cast<const uint4*>(tv.dterms + h.d0 + (int64_t)tid * h.KD);
+  const uint4 pad4 = make_uint4(m | m << 16, m | m << 16, m | m << 16, m | m << 16);
+  uint4 dq[3] = {pad4, pad4, pad4};
+  if (tid < R) {
 #pragma unroll
     for (int u = 0; u < 3; u++)
-      if (8 * u < KD) dq[u] = __ldg(dv + u);
+      if (8 * u < h.KD) dq[u] = __ldg(dv + u);
   }
-  const int eb = __ldg(tv.edge_ptr + t), ne = __ldg(tv.edge_ptr + t + 1) - eb;
-  const int tb = __ldg(tv.eterm_ptr + t);
-  const int KE = ne ? (__ldg(tv.eterm_ptr + t + 1) - tb) / ne : 0;
-  // the diagonal threads take the last edges of a round, the others the first
   const int q0 = (tid >= R) ? tid - R : T - R + tid;
+  auto eterm8 = [&](int q, int g) {
+    return __ldg(reinterpret_cast<const uint4*>(tv.eterms + h.t0 + (int64_t)q * h.KE) + g);
+  };
   int2 ep[2];
-  uint4 eq[2] = {none4, none4};
+  uint4 eq[2] = {pad4, pad4};
 #pragma unroll
   for (int u = 0; u < 2; u++) {
     const int q = q0 + u * T;
-    if (q < ne) {
-      ep[u] = __ldg(tv.edge_pos + eb + q);
-      eq[u] = __ldg(reinterpret_cast<const uint4*>(tv.eterms + tb + (int64_t)q * KE));
+    if (q < h.ne) {
+      ep[u] = __ldg(tv.edge_pos + h.e0 + q);
+      if (h.KE) eq[u] = eterm8(q, 0);
     }
   }
-  // ... and each thread turns the records it copied into element entries in place
+  // ... the copies ...
+  auto copy_cell = [&](int i, int32_t c) {  // the thread's own cell: De, alpha
+    double* slot = E + (size_t)i * TILE_EW;
+    if (MODE != TP_ASM_MASS) cp_async<8>(slot + 8, De + c);
+    if (MODE == TP_ASM_FULL && alpha) cp_async<8>(slot + 9, alpha + c);
+    if constexpr (DIAG && !CMP) {
+      if (ex.alpha)
+        for (int s = 0; s < ex.S; s++)
+          cp_async<8>(X + (size_t)i * nd + s, ex.alpha + (int64_t)c * ex.ld + s);
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < MAXC; u++) {
+    const int ib = (tid & ~31) + u * T;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (cq[u][k] >= 0)
+        cp_async<16>(E + (ib + (lane >> 2) + 8 * k) * TILE_EW + 2 * (lane & 3),
+                     geo + 8 * (int64_t)cq[u][k] + 2 * (lane & 3));
+    if (cid[u] >= 0) copy_cell(ib + lane, cid[u]);
+  }
+  for (int ib = (tid & ~31) + MAXC * T; ib < m; ib += T) {  // tiles of more than MAXC T cells
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int j = ib + (lane >> 2) + 8 * k;
+      if (j < m)
+        cp_async<16>(E + j * TILE_EW + 2 * (lane & 3),
+                     geo + 8 * (int64_t)__ldg(ids + j) + 2 * (lane & 3));
+    }
+    if (ib + lane < m) copy_cell(ib + lane, __ldg(ids + ib + lane));
+  }
+  if (tid < TILE_EW) E[m * TILE_EW + tid] = 0.0;
+  // ... and each warp turns the records it copied into element entries in place
   cp_async_wait_all();
+  __syncwarp();
   for (int i = tid; i < m; i += T)
-    tile_cell_entries<MODE, DIAG, CMP>(E + (size_t)i * ew, alpha != nullptr, inv_dt, lumped, ex,
-                                       dsh);
+    tile_cell_entries<MODE, DIAG, CMP>(E + (size_t)i * TILE_EW, X + (size_t)i * nd,
+                                       alpha != nullptr, inv_dt, lumped, ex, dsh);
   __syncthreads();
 
   // ---- phase B1: the diagonal of each tile row
@@ -381,29 +368,34 @@ __global__ void __launch_bounds__(TILE_BLOCK, 3) k_assemble_tiles(
     const bool is_bc = bc_mask && bc_mask[r];
     double dacc = 0.0, dg[4] = {0.0, 0.0, 0.0, 0.0};
     if (!is_bc) {
-      auto group = [&](const uint4& g8) -> bool {
+      auto lumped_terms = [&](const uint4& g8) {
+        if constexpr (DIAG) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const uint32_t tm = term_of(g8, k);
-          if (tm == TILE_TERM_NONE) return false;
-          const int loc = tm & ((1 << TILE_LOC_BITS) - 1), li = tm >> TILE_LOC_BITS;
-          const double* e = E + (size_t)loc * ew;
-          dacc = __dadd_rn(dacc, e[tri_index(li, li)]);
-          if constexpr (DIAG && CMP) {
-            // the term tile_cell_entries forms without per-cell alpha, (shift_s + 0) Ld
+          for (int k = 0; k < 8; k++) {
+            const int loc = term_of(g8, k) & TILE_LOC_MASK;
+            const bool real = loc != m;
+            const double* x = X + (size_t)(real ? loc : 0) * nd;
 #pragma unroll
-            for (int s = 0; s < 4; s++)
-              if (s < ex.S) dg[s] = __dadd_rn(dg[s], __dmul_rn(__dadd_rn(dsh[s], 0.0), e[10]));
-          } else if constexpr (DIAG) {
-#pragma unroll
-            for (int s = 0; s < 4; s++)
-              if (s < ex.S) dg[s] = __dadd_rn(dg[s], e[10 + s]);
+            for (int s = 0; s < 4; s++) {
+              if (s >= ex.S) break;
+              // without per-cell alpha the term tile_cell_entries forms, (shift_s + 0) Ld
+              const double v = CMP ? __dmul_rn(__dadd_rn(dsh[s], 0.0), x[0]) : x[s];
+              if (real) dg[s] = __dadd_rn(dg[s], v);
+            }
           }
         }
-        return true;
       };
-      bool more = group(dq[0]) && group(dq[1]) && group(dq[2]);
-      for (int g = 3; more && 8 * g < KD; g++) more = group(__ldg(dv + g));
+#pragma unroll
+      for (int g = 0; g < 3; g++)
+        if (8 * g < h.KD) {
+          dacc = add_terms(E, dq[g], dacc);
+          lumped_terms(dq[g]);
+        }
+      for (int g = 3; 8 * g < h.KD; g++) {
+        const uint4 d = __ldg(dv + g);
+        dacc = add_terms(E, d, dacc);
+        lumped_terms(d);
+      }
     }
     const double v = is_bc ? 1.0 : dacc;
     // a vertex no cell uses has an empty row (pd = -1)
@@ -432,23 +424,11 @@ __global__ void __launch_bounds__(TILE_BLOCK, 3) k_assemble_tiles(
 
   // ---- phase B2: the tile's edges, (r, v) and (v, r) from one ordered sum
   auto edge = [&](int q, int2 pp, const uint4& g0) {
-    double acc = 0.0;
-    auto group = [&](const uint4& g8) -> bool {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t tm = term_of(g8, k);
-        if (tm == TILE_TERM_NONE) return false;
-        const int loc = tm & ((1 << TILE_LOC_BITS) - 1), tq = tm >> TILE_LOC_BITS;
-        acc = __dadd_rn(acc, E[(size_t)loc * ew + tq]);
-      }
-      return true;
-    };
-    bool more = group(g0);
-    for (int g = 1; more && 8 * g < KE; g++)
-      more = group(__ldg(reinterpret_cast<const uint4*>(tv.eterms + tb + (int64_t)q * KE) + g));
+    double acc = add_terms(E, g0, 0.0);
+    for (int g = 1; 8 * g < h.KE; g++) acc = add_terms(E, eterm8(q, g), acc);
     double a_rv = acc, a_vr = acc;
     if (bc_mask || ex.sell32) {
-      const int2 rv = __ldg(tv.edge_rv + eb + q);
+      const int2 rv = __ldg(tv.edge_rv + h.e0 + q);
       if (bc_mask) {
         if (bc_mask[rv.x]) a_rv = 0.0;
         if (bc_mask[rv.y]) a_vr = 0.0;
@@ -467,11 +447,10 @@ __global__ void __launch_bounds__(TILE_BLOCK, 3) k_assemble_tiles(
       out32[pp.y] = (float)a_vr;
     }
   };
-  if (q0 < ne) edge(q0, ep[0], eq[0]);
-  if (q0 + T < ne) edge(q0 + T, ep[1], eq[1]);
-  for (int q = q0 + 2 * T; q < ne; q += T)
-    edge(q, __ldg(tv.edge_pos + eb + q),
-         __ldg(reinterpret_cast<const uint4*>(tv.eterms + tb + (int64_t)q * KE)));
+  if (q0 < h.ne) edge(q0, ep[0], eq[0]);
+  if (q0 + T < h.ne) edge(q0 + T, ep[1], eq[1]);
+  for (int q = q0 + 2 * T; q < h.ne; q += T)
+    edge(q, __ldg(tv.edge_pos + h.e0 + q), h.KE ? eterm8(q, 0) : pad4);
   if (ex.sell32 && t == 0 && (nv & 31)) {
     // the lanes of the last slice past the last row: padding, 0
     const int64_t sl = nv >> 5;
@@ -638,86 +617,41 @@ __host__ __device__ inline int rhs_slot_width(bool lumped, int S, bool f) {
   return lumped ? 1 : (2 + (f ? 2 : 1) * S) | 1;
 }
 
-template <bool LUMPED>
-__global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
-                                                   const int32_t* __restrict__ cells,
-                                                   const double* __restrict__ geo,
-                                                   const double* __restrict__ u,
-                                                   const double* __restrict__ f, double inv_dt,
-                                                   double* __restrict__ b) {
+// SC: columns held (1 or 4; S <= SC).
+template <bool LUMPED, int SC>
+__global__ void __launch_bounds__(256, SC == 1 ? 4 : 3) k_rhs_tiles(
+    TileView tv, int S, int ld, const int32_t* __restrict__ cells,
+    const double* __restrict__ geo, const double* __restrict__ u, const double* __restrict__ f,
+    double inv_dt, double* __restrict__ b) {
   extern __shared__ double sm_ld[];
-  const int R = tv.R, T = blockDim.x, t = blockIdx.x, tid = threadIdx.x;
-  const int c0 = __ldg(tv.cell_ptr + t), m = __ldg(tv.cell_ptr + t + 1) - c0;
-  const int CW = rhs_slot_width(LUMPED, S, f != nullptr), FO = 2 + S;
-  {
-    constexpr int MAXC = 4;
-    int64_t cid[MAXC];
-    double dj[MAXC];
-    int4 cv[MAXC];
-#pragma unroll
-    for (int k = 0; k < MAXC; k++) {
-      const int i = tid + k * T;
-      cid[k] = (i < m) ? (int64_t)__ldg(tv.cells + c0 + i) : -1;
-    }
-#pragma unroll
-    for (int k = 0; k < MAXC; k++) {
-      dj[k] = (cid[k] >= 0) ? __ldg(geo + 8 * cid[k] + 6) : 0.0;
-      if constexpr (!LUMPED)
-        cv[k] = (cid[k] >= 0) ? __ldg(reinterpret_cast<const int4*>(cells) + cid[k])
-                              : make_int4(0, 0, 0, 0);
-    }
-    auto put = [&](int i, double djv, const int4& c4) {
-      double* slot = sm_ld + (size_t)i * CW;
-      if constexpr (LUMPED) {
-        slot[0] = __dmul_rn(div120(djv), 5.0);
-      } else {
-        const double base = div120(djv);
-        slot[0] = __dmul_rn(base, inv_dt);
-        slot[1] = base;
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-          if (s >= S) break;
-          slot[2 + s] = __dadd_rn(
-              __dadd_rn(__dadd_rn(__ldg(u + (int64_t)c4.x * ld + s), __ldg(u + (int64_t)c4.y * ld + s)),
-                        __ldg(u + (int64_t)c4.z * ld + s)),
-              __ldg(u + (int64_t)c4.w * ld + s));
-          if (f)
-            slot[FO + s] = __dadd_rn(
-                __dadd_rn(__dadd_rn(__ldg(f + (int64_t)c4.x * ld + s), __ldg(f + (int64_t)c4.y * ld + s)),
-                          __ldg(f + (int64_t)c4.z * ld + s)),
-                __ldg(f + (int64_t)c4.w * ld + s));
-        }
-      }
-    };
-#pragma unroll
-    for (int k = 0; k < MAXC; k++)
-      if (cid[k] >= 0) put(tid + k * T, dj[k], cv[k]);
-    for (int i = tid + MAXC * T; i < m; i += T) {
-      const int64_t c = __ldg(tv.cells + c0 + i);
-      put(i, __ldg(geo + 8 * c + 6),
-          LUMPED ? make_int4(0, 0, 0, 0) : __ldg(reinterpret_cast<const int4*>(cells) + c));
-    }
-  }
-  // the row's first 24 terms and its u, f are loaded before the barrier (in flight with
-  // the loads above)
+  constexpr int T = 256;
+  const int R = tv.R, t = blockIdx.x, tid = threadIdx.x;
   int64_t r = -1;
-  double w[4] = {0.0, 0.0, 0.0, 0.0}, fr[4] = {0.0, 0.0, 0.0, 0.0};
-  const uint4* dv = nullptr;
-  int KD = 0;
-  const uint4 none4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-  uint4 dq[3] = {none4, none4, none4};
+  if (tid < R) r = __ldg(tv.rows + (int64_t)t * R + tid);
+  const TileHead h = tile_head(tv, t);
+  const int m = h.m;
+  const int CW = rhs_slot_width(LUMPED, S, f != nullptr), FO = 2 + S;
+  constexpr int MAXC = 4;
+  int32_t cid[MAXC];
+#pragma unroll
+  for (int k = 0; k < MAXC; k++) {
+    const int i = tid + k * T;
+    cid[k] = (i < m) ? __ldg(tv.cells + h.c0 + i) : -1;
+  }
+  // the row's first 24 terms and its u, f (in flight with the cells' loads)
+  double w[SC], fr[SC];
+  const uint4* const dv = reinterpret_cast<const uint4*>(tv.dterms + h.d0 + (int64_t)tid * h.KD);
+  uint4 dq[3];
+#pragma unroll
+  for (int s = 0; s < SC; s++) w[s] = fr[s] = 0.0;
   if (tid < R) {
-    r = __ldg(tv.rows + (int64_t)t * R + tid);
-    const int d0 = __ldg(tv.dterm_ptr + t);
-    KD = (__ldg(tv.dterm_ptr + t + 1) - d0) / R;
-    dv = reinterpret_cast<const uint4*>(tv.dterms + d0 + (int64_t)tid * KD);
 #pragma unroll
     for (int g = 0; g < 3; g++)
-      if (8 * g < KD) dq[g] = __ldg(dv + g);
+      if (8 * g < h.KD) dq[g] = __ldg(dv + g);
     if (r >= 0) {
 #pragma unroll
-      for (int s = 0; s < 4; s++) {
-        if (s >= S) continue;
+      for (int s = 0; s < SC; s++) {
+        if (s >= S) break;
         if constexpr (LUMPED) {
           w[s] = __dadd_rn(__dmul_rn(inv_dt, u[r * ld + s]), f ? f[r * ld + s] : 0.0);
         } else {
@@ -727,38 +661,85 @@ __global__ void __launch_bounds__(256) k_rhs_tiles(TileView tv, int S, int ld,
       }
     }
   }
+  {
+    double dj[MAXC];
+    int4 cv[MAXC];
+#pragma unroll
+    for (int k = 0; k < MAXC; k++) {
+      dj[k] = (cid[k] >= 0) ? __ldg(geo + 8 * (int64_t)cid[k] + 6) : 0.0;
+      if constexpr (!LUMPED)
+        cv[k] = (cid[k] >= 0) ? __ldg(reinterpret_cast<const int4*>(cells) + cid[k])
+                              : make_int4(0, 0, 0, 0);
+    }
+    auto put = [&](int i, double djv, const int4& c4) {
+      double* slot = sm_ld + (size_t)i * CW;
+      if constexpr (LUMPED) {
+        slot[0] = __dmul_rn(div120(djv), 5.0);
+      } else {
+        auto vertex_sum = [&](const double* __restrict__ x, int s) {
+          const double x0 = __ldg(x + (int64_t)c4.x * ld + s), x1 = __ldg(x + (int64_t)c4.y * ld + s),
+                       x2 = __ldg(x + (int64_t)c4.z * ld + s), x3 = __ldg(x + (int64_t)c4.w * ld + s);
+          return __dadd_rn(__dadd_rn(__dadd_rn(x0, x1), x2), x3);
+        };
+        const double base = div120(djv);
+        slot[0] = __dmul_rn(base, inv_dt);
+        slot[1] = base;
+#pragma unroll
+        for (int s = 0; s < SC; s++) {
+          if (s >= S) break;
+          slot[2 + s] = vertex_sum(u, s);
+          if (f) slot[FO + s] = vertex_sum(f, s);
+        }
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < MAXC; k++)
+      if (cid[k] >= 0) put(tid + k * T, dj[k], cv[k]);
+    for (int i = tid + MAXC * T; i < m; i += T) {
+      const int64_t c = __ldg(tv.cells + h.c0 + i);
+      put(i, __ldg(geo + 8 * c + 6),
+          LUMPED ? make_int4(0, 0, 0, 0) : __ldg(reinterpret_cast<const int4*>(cells) + c));
+    }
+  }
   __syncthreads();
   if (r < 0) return;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  auto group = [&](const uint4& g8) -> bool {
+  double acc[SC];
+#pragma unroll
+  for (int s = 0; s < SC; s++) acc[s] = 0.0;
+  // 8 terms: their slots' reads in flight together; padding terms (loc = m) add nothing
+  auto group = [&](const uint4& g8) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      const uint32_t tm = term_of(g8, k);
-      if (tm == TILE_TERM_NONE) return false;
-      const double* slot = sm_ld + (size_t)(tm & ((1 << TILE_LOC_BITS) - 1)) * CW;
+      const int loc = term_of(g8, k) & TILE_LOC_MASK;
+      const bool real = loc != m;
+      const double* slot = sm_ld + (size_t)(real ? loc : 0) * CW;
       if constexpr (LUMPED) {
         const double Ld = slot[0];
 #pragma unroll
-        for (int s = 0; s < 4; s++)
-          if (s < S) acc[s] = __dadd_rn(acc[s], __dmul_rn(Ld, w[s]));
+        for (int s = 0; s < SC; s++) {
+          const double v = __dmul_rn(Ld, w[s]);
+          if (real) acc[s] = __dadd_rn(acc[s], v);
+        }
       } else {
         const double mdt = slot[0], base = slot[1];
 #pragma unroll
-        for (int s = 0; s < 4; s++) {
-          if (s >= S) continue;
+        for (int s = 0; s < SC; s++) {
+          if (SC > 1 && s >= S) break;
           const double sf = f ? slot[FO + s] : 0.0;
-          acc[s] = __dadd_rn(acc[s], __dadd_rn(__dmul_rn(mdt, __dadd_rn(slot[2 + s], w[s])),
-                                               __dmul_rn(base, __dadd_rn(sf, fr[s]))));
+          const double v = __dadd_rn(__dmul_rn(mdt, __dadd_rn(slot[2 + s], w[s])),
+                                     __dmul_rn(base, __dadd_rn(sf, fr[s])));
+          if (real) acc[s] = __dadd_rn(acc[s], v);
         }
       }
     }
-    return true;
   };
-  bool more = group(dq[0]) && group(dq[1]) && group(dq[2]);
-  for (int g = 3; more && 8 * g < KD; g++) more = group(__ldg(dv + g));
+#pragma unroll
+  for (int g = 0; g < 3; g++)
+    if (8 * g < h.KD) group(dq[g]);
+  for (int g = 3; 8 * g < h.KD; g++) group(__ldg(dv + g));
 #pragma unroll
   for (int s = 0; s < 4; s++)
-    if (s < ld) b[r * ld + s] = (s < S) ? acc[s] : 0.0;
+    if (s < ld) b[r * ld + s] = (s < SC && s < S) ? acc[s < SC ? s : 0] : 0.0;
 }
 
 // lumped right-hand side from the per-vertex lumped mass: b = m (inv_dt u + f) per column
@@ -1188,11 +1169,10 @@ static int launch_tiles(const tp_mesh* m, const double* De, const double* alpha,
   *used = false;
   if (!m->tiles) return TP_OK;
   const TileView& tv = m->tiles->v;
-  // slot of 5 or 7 sixteen-byte units (tile_cell_entries), or 11 doubles for DIAG without
-  // per-cell alpha (three CTAs of the largest tiles per SM instead of two)
+  // DIAG: the cell's lumped factor, or its S column terms when alpha differs per cell
   const bool cmp = DIAG && ex.alpha == nullptr;
-  const int ew = DIAG ? (cmp ? 11 : 14) : 10;
-  const size_t smem = sizeof(double) * (size_t)tv.max_cells * ew;
+  const int nd = DIAG ? (cmp ? 1 : ex.S) : 0;
+  const size_t smem = sizeof(double) * (size_t)(tv.max_cells + 1) * (TILE_EW + nd);
   int dev = 0, optin = 0;
   TP_CUDA_TRY(cudaGetDevice(&dev));
   TP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -1207,7 +1187,7 @@ static int launch_tiles(const tp_mesh* m, const double* De, const double* alpha,
     TP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      (int)cudaSharedmemCarveoutMaxShared));
   fn<<<tv.n_tiles, TILE_BLOCK, smem, st>>>(tv, m->geo, De, alpha, inv_dt, lumped, bc_mask,
-                                           m->indptr, out64, out32, ex, ew, m->n_verts);
+                                           m->indptr, out64, out32, ex, nd, m->n_verts);
   TP_LAUNCH_CHECK();
   *used = true;
   return TP_OK;
@@ -1348,7 +1328,8 @@ extern "C" int tp_assemble_rhs(const tp_mesh* m, int S, int ld, const double* u_
   if (m->n_verts > 0 && m->tiles && m->tiles->v.n_tiles > 0 && m->tiles->v.R <= 256 &&
       smem_t <= (size_t)optin) {
     const TileView& tv = m->tiles->v;
-    auto fn = lumped ? k_rhs_tiles<true> : k_rhs_tiles<false>;
+    auto fn = S == 1 ? (lumped ? k_rhs_tiles<true, 1> : k_rhs_tiles<false, 1>)
+                     : (lumped ? k_rhs_tiles<true, 4> : k_rhs_tiles<false, 4>);
     if (smem_t > 48 * 1024)
       TP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
     fn<<<tv.n_tiles, 256, smem_t, st>>>(tv, S, ld, m->cells, m->geo, u_old, f, inv_dt, b);

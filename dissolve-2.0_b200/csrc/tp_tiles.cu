@@ -391,7 +391,7 @@ struct TileBuild {
   int32_t *rows, *diag_pos, *cells;
   uint16_t *dterms, *eterms;
   int2 *edge_pos, *edge_rv;
-  const int32_t *cell_ptr, *dterm_ptr, *edge_ptr, *eterm_ptr;
+  const TileHead* head;
 };
 
 constexpr int TB_T = 256;
@@ -510,21 +510,26 @@ __global__ void __launch_bounds__(TB_T) k_tile_build(TileBuild b) {
   __syncthreads();
   const int KD = (s_kmax + 7) & ~7;
   if constexpr (FILL) {
-    const int c0 = b.cell_ptr[t];
-    for (int i = tid; i < m; i += TB_T) b.cells[c0 + i] = s_tc[i];
+    const TileHead h = b.head[t];
+    for (int i = tid; i < m; i += TB_T) b.cells[h.c0 + i] = s_tc[i];
     // local index of every visit and the diagonal terms [row][k]
-    uint16_t* dt = b.dterms + b.dterm_ptr[t];
+    uint16_t* dt = b.dterms + h.d0;
+    for (int k = tid; k < KD * b.R; k += TB_T) dt[k] = (uint16_t)m;
+    for (int k = tid; k < h.KE * nedge; k += TB_T) b.eterms[h.t0 + k] = (uint16_t)m;
+    __syncthreads();
     for (int k = tid; k < nvis; k += TB_T) {
       const int i = row_of(k);
       const int32_t e = b.v2c[b.vptr[s_row[i]] + (k - s_vis[i])];
       const int loc = lower_bound(s_tc, 0, m, e >> 2);
       s_loc[k] = (uint16_t)loc;
-      dt[(int64_t)i * KD + (k - s_vis[i])] = (uint16_t)(loc | ((e & 3) << TILE_LOC_BITS));
+      const int li = e & 3;
+      const int tri = li * (9 - li) / 2;  // 0, 4, 7, 9
+      dt[(int64_t)i * KD + (k - s_vis[i])] = (uint16_t)(loc | (tri << TILE_LOC_BITS));
     }
     __syncthreads();
   }
   // edge terms: each row's thread walks its cells in ascending order
-  const int KE = FILL && nedge ? (b.eterm_ptr[t + 1] - b.eterm_ptr[t]) / nedge : 0;
+  const int t0 = FILL ? b.head[t].t0 : 0, KE = FILL ? b.head[t].KE : 0;
   if (tid < nr) {
     const int32_t r = s_row[tid];
     const int v0 = b.vptr[r], deg = b.vptr[r + 1] - v0, len = b.indptr[r + 1] - b.indptr[r];
@@ -550,7 +555,7 @@ __global__ void __launch_bounds__(TB_T) k_tile_build(TileBuild b) {
         if constexpr (FILL) {
           const int a = li < j ? li : j, c = li < j ? j : li;
           const int tri = (a == 0 ? 0 : (a == 1 ? 4 : 7)) + (c - a);
-          b.eterms[b.eterm_ptr[t] + (int64_t)e * KE + q] =
+          b.eterms[t0 + (int64_t)e * KE + q] =
               (uint16_t)(s_loc[s_vis[tid] + k] | (tri << TILE_LOC_BITS));
         }
       }
@@ -561,9 +566,9 @@ __global__ void __launch_bounds__(TB_T) k_tile_build(TileBuild b) {
   if constexpr (!FILL) {
     if (tid == 0)
       b.sizes[t] = s_bad ? make_int4(0, 0, 0, 0)
-                         : make_int4(m, KD * b.R, nedge, ((s_kemax + 7) & ~7) * nedge);
+                         : make_int4(m, KD, nedge, nedge ? (s_kemax + 7) & ~7 : 0);
   } else {
-    const int eb = b.edge_ptr[t];
+    const int eb = b.head[t].e0;
     for (int e = tid; e < nedge; e += TB_T) {
       int lo = 0, hi = nr;  // the row that owns edge e
       while (hi - lo > 1) {
@@ -766,24 +771,20 @@ extern "C" int tp_tiles_create(const tp_mesh* m, int rows_per_tile, void* stream
   }
   int rc = check();
   if (rc) return rc;
-  std::vector<int32_t> cell_ptr(nt + 1, 0), dterm_ptr(nt + 1, 0), edge_ptr(nt + 1, 0),
-      eterm_ptr(nt + 1, 0);
+  std::vector<TileHead> head(nt);
   int64_t tc = 0, td = 0, te = 0, tt = 0;
   int max_cells = 0, max_edges = 0;
   for (int t = 0; t < nt; t++) {
     const int4 z = h_sizes[t];
+    head[t] = {(int32_t)tc, z.x, (int32_t)td, z.y, (int32_t)te, z.z, (int32_t)tt, z.w};
     tc += z.x;
-    td += z.y;
+    td += (int64_t)z.y * R;
     te += z.z;
-    tt += z.w;
+    tt += (int64_t)z.w * z.z;
     if (tc > INT32_MAX || td > INT32_MAX || te > INT32_MAX || tt > INT32_MAX) {
       set_error("tile terms exceed int32 offsets");
       return TP_ERR_CAPACITY;
     }
-    cell_ptr[t + 1] = (int32_t)tc;
-    dterm_ptr[t + 1] = (int32_t)td;
-    edge_ptr[t + 1] = (int32_t)te;
-    eterm_ptr[t + 1] = (int32_t)tt;
     max_cells = std::max(max_cells, z.x);
     max_edges = std::max(max_edges, z.z);
   }
@@ -794,12 +795,10 @@ extern "C" int tp_tiles_create(const tp_mesh* m, int rows_per_tile, void* stream
     ~Guard() { delete h; }
   } guard{h};
   off = 0;
-  const size_t o_rows = take(4 * (size_t)nt * R), o_dpos = take(4 * (size_t)nt * R),
-               o_cptr = take(4 * (size_t)(nt + 1)), o_cells = take(4 * (size_t)tc),
-               o_dptr = take(4 * (size_t)(nt + 1)), o_dterms = take(2 * (size_t)td),
-               o_eptr = take(4 * (size_t)(nt + 1)), o_epos = take(8 * (size_t)te),
-               o_erv = take(8 * (size_t)te), o_tptr = take(4 * (size_t)(nt + 1)),
-               o_eterms = take(2 * (size_t)tt);
+  const size_t o_head = take(sizeof(TileHead) * (size_t)nt), o_rows = take(4 * (size_t)nt * R),
+               o_dpos = take(4 * (size_t)nt * R), o_cells = take(4 * (size_t)tc),
+               o_dterms = take(2 * (size_t)td), o_epos = take(8 * (size_t)te),
+               o_erv = take(8 * (size_t)te), o_eterms = take(2 * (size_t)tt);
   h->bytes = off;
   cudaError_t ce = cudaMalloc(&h->dmem, h->bytes);
   if (ce != cudaSuccess) {
@@ -827,18 +826,10 @@ extern "C" int tp_tiles_create(const tp_mesh* m, int rows_per_tile, void* stream
   v.edge_pos = b.edge_pos;
   v.edge_rv = b.edge_rv;
   v.eterms = b.eterms;
-  v.cell_ptr = b.cell_ptr = reinterpret_cast<int32_t*>(p + o_cptr);
-  v.dterm_ptr = b.dterm_ptr = reinterpret_cast<int32_t*>(p + o_dptr);
-  v.edge_ptr = b.edge_ptr = reinterpret_cast<int32_t*>(p + o_eptr);
-  v.eterm_ptr = b.eterm_ptr = reinterpret_cast<int32_t*>(p + o_tptr);
-  const size_t pb = 4 * (size_t)(nt + 1);
-  TP_CUDA_TRY(cudaMemcpyAsync(p + o_cptr, cell_ptr.data(), pb, cudaMemcpyHostToDevice, st));
-  TP_CUDA_TRY(cudaMemcpyAsync(p + o_dptr, dterm_ptr.data(), pb, cudaMemcpyHostToDevice, st));
-  TP_CUDA_TRY(cudaMemcpyAsync(p + o_eptr, edge_ptr.data(), pb, cudaMemcpyHostToDevice, st));
-  TP_CUDA_TRY(cudaMemcpyAsync(p + o_tptr, eterm_ptr.data(), pb, cudaMemcpyHostToDevice, st));
-  // unused terms are TILE_TERM_NONE
-  TP_CUDA_TRY(cudaMemsetAsync(p + o_dterms, 0xff, 2 * (size_t)td, st));
-  TP_CUDA_TRY(cudaMemsetAsync(p + o_eterms, 0xff, 2 * (size_t)tt, st));
+  v.head = b.head = reinterpret_cast<TileHead*>(p + o_head);
+  if (nt)
+    TP_CUDA_TRY(cudaMemcpyAsync(p + o_head, head.data(), sizeof(TileHead) * (size_t)nt,
+                                cudaMemcpyHostToDevice, st));
   if (nt) {
     k_tile_build<true><<<nt, TB_T, smem, st>>>(b);
     TP_LAUNCH_CHECK();
