@@ -371,6 +371,13 @@ def roofline_solve(fast, flush, torch):
                   "iteration, values and vectors in tensor memory, one cooperative launch "
                   "per solve)")
         engine = "k_pcgp"
+    elif window and "exchange" in form:
+        # exchange engine: the same count
+        bytes_it = nnz * 4 + 12 * nv * 16
+        kernel = ("k_ccg<float,4,3,4,true> (persistent 3-column Jacobi-PCG on every SM, "
+                  "Chronopoulos-Gear form, vectors in registers, values in tensor memory, data "
+                  "exchanged with its pass number, one cooperative launch per solve)")
+        engine = "k_ccg"
     elif window:
         # window engine, per iteration: FP32 value per nonzero (columns stay in shared
         # memory for the whole solve) and 12 passes of (V, 4) FP32: u read once into the
@@ -405,7 +412,7 @@ def roofline_solve(fast, flush, torch):
             "note": f"peak = HBM copy bandwidth ({peak_src}); one solve of the current "
                     "state from the previous-step guess; the operator and vectors stay on "
                     "chip (tensor memory, shared memory) and in the 126 MB L2 between "
-                    "iterations, so the solve is bound by its grid barrier and on-chip "
+                    "iterations, so the solve is bound by its exchanges and on-chip "
                     "latencies, not by DRAM; traffic = ncu DRAM bytes per iteration x "
                     "iterations of this launch"}
 

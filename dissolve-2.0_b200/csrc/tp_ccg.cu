@@ -35,6 +35,14 @@
 // 4 lane + k % 4: four columns per 8-byte load; slices are at least 16 entries wide, so
 // that those in tensor memory have fixed addresses.  Dot products are FP64 partials summed in CTA order:
 // results depend on the cluster size only, which is fixed at create.
+// A system past one cluster runs the same passes on every SM (GRID): the exchanges then go
+// through L2, and again no barrier is needed per iteration, because the data carries its own
+// flag.  Every row of u is published in 16-byte units that hold values and the pass number
+// (a unit is written and read in one access), and a CTA polls the units of its halo and the
+// partial sums of the others until their number is this pass': one store and one load of
+// latency per exchange, where a grid barrier costs an arrival, a poll and then the load.
+// The buffers are cleared before a solve, so an old number is never taken for a new one; a
+// unit is rewritten only after its readers have sent the sums that the writer waits for.
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -83,6 +91,12 @@ struct CcgArgs {
   const double* rtol;
   CcgOut* out;
   int win_cap, dyn_bytes;
+  // GRID: halo rows of every part, published rows (16-byte units), partial sums (units of
+  // two buffers x CTA x 16), arrivals of the grid barrier around the FP64 sweeps
+  const int32_t* halo;
+  ulonglong2* ubuf;
+  ulonglong2* sums;
+  unsigned int* bar;
   unsigned long long wait_limit_ns;
   unsigned int wait_missing;  // > 0 (tests): every wait expects that many bytes too many
 };
@@ -190,6 +204,46 @@ __device__ __forceinline__ bool mb_wait(uint64_t* mb, uint32_t parity,
   while (!mb_try(mb, parity))
     if (cc_time() - t0 > limit_ns) return false;
   return true;
+}
+
+// 16 bytes in one access (GRID exchanges)
+__device__ __forceinline__ void st_unit(ulonglong2* p, unsigned long long lo,
+                                        unsigned long long hi) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"(lo), "l"(hi)
+      : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_unit(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\t"
+      "mov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(v.x), "=l"(v.y)
+      : "l"(p)
+      : "memory");
+  return v;
+}
+// a unit whose number is not `want` yet: polled until it is, false after limit_ns or once
+// another thread of the CTA gave up
+template <int SHIFT>
+__device__ __forceinline__ bool poll_unit(const ulonglong2* p, ulonglong2& v, uint32_t want,
+                                          unsigned long long limit_ns, const volatile int* gave_up) {
+  if ((uint32_t)(v.y >> SHIFT) == want) return true;
+  unsigned long long t0 = 0;
+  for (unsigned n = 0;; n++) {
+    v = ld_unit(p);
+    if ((uint32_t)(v.y >> SHIFT) == want) return true;
+    if ((n & 15u) == 15u) {
+      if (*gave_up) return false;
+      const unsigned long long t = cc_time();
+      if (t0 == 0)
+        t0 = t;
+      else if (t - t0 > limit_ns)
+        return false;
+    }
+  }
 }
 
 // tensor memory: 16 consecutive 32-bit columns of this thread's lane
@@ -330,7 +384,7 @@ __device__ __forceinline__ void axpy_row(VT v, const VT u[LD], VT y[LD]) {
 // sums (16 CTAs x 16), the window (win_cap rows), w, then this part's slice offsets, push
 // list, diagonal, columns and values, each where it still fits.
 // NC: columns computed (S <= NC <= LD).
-template <typename VT, int LD, int NC, int RPT>
+template <typename VT, int LD, int NC, int RPT, bool GRID>
 __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   double* const s_part = reinterpret_cast<double*>(s_dyn);  // [2][rank][quantity * 4 + column]
@@ -346,8 +400,51 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   constexpr int RB = LD * (int)sizeof(VT);
   constexpr int VW = (int)sizeof(VT) / 4;             // 32-bit words of a value
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t rank = cl_rank(), C = cl_size();
+  const uint32_t rank = GRID ? blockIdx.x : cl_rank(), C = GRID ? gridDim.x : cl_size();
   const int S = a.S;
+  // GRID: 16-byte units of a published row, and where a unit keeps its pass number
+  constexpr int UW = sizeof(VT) == 8 ? NC : (NC + 2) / 3;
+  constexpr int TAG = sizeof(VT) == 8 ? 0 : 32;
+  uint32_t epoch = 1, arrivals = 0;
+  auto x_sync = [&]() {  // x written by every CTA of the system is visible to all
+    if constexpr (!GRID) {
+      cl_sync();
+    } else {
+      __syncthreads();
+      if (tid == 0) {
+        arrivals += C + a.wait_missing;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+        const unsigned long long t0 = cc_time();
+        for (;;) {
+          uint32_t v;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+          if ((int)(v - arrivals) >= 0) break;
+          if (cc_time() - t0 > a.wait_limit_ns) {
+            s_gave_up = 1;
+            break;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  };
+  // GRID: this pass' u of a row for the CTAs that hold it as halo
+  auto publish = [&](int64_t row, const VT* uv) {
+    if constexpr (GRID) {
+#pragma unroll
+      for (int k = 0; k < UW; k++) {
+        if constexpr (sizeof(VT) == 8) {
+          st_unit(a.ubuf + row * UW + k, (unsigned long long)__double_as_longlong(uv[k]), epoch);
+        } else {
+          auto w = [&](int s) {
+            return (unsigned long long)(s < NC ? __float_as_uint(uv[s < NC ? s : 0]) : 0u);
+          };
+          st_unit(a.ubuf + row * UW + k, w(3 * k) | w(3 * k + 1) << 32,
+                  w(3 * k + 2) | (unsigned long long)epoch << 32);
+        }
+      }
+    }
+  };
   if (warp == 0) cc_tm_alloc(&s_taddr);
   if (tid == 0) {
     s_gave_up = 0;
@@ -355,15 +452,18 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  cl_sync();
+  if constexpr (GRID)
+    __syncthreads();
+  else
+    cl_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tm = s_taddr + ((uint32_t)(32 * (warp & 3)) << 16) + 128u * (uint32_t)(warp >> 2);
   uint32_t ph_part = 0, ph_halo = 0;  // mbarrier phases: bit b of ph_part for buffer b
   uint32_t buf = 0;
   bool alive = true;
   {
-    const int sys = a.order[cl_id()];
-    const CcgPart part = a.parts[(int64_t)cl_id() * C + rank];
+    const int sys = GRID ? 0 : a.order[cl_id()];
+    const CcgPart part = a.parts[GRID ? (int64_t)rank : (int64_t)cl_id() * C + rank];
     const int nrows = part.nrows;
     const int64_t row0 = part.row0;
     // ---- this part's tables: byte offsets into s_dyn, 16-byte granules; -1: no room (the
@@ -378,12 +478,14 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     };
     VT* const s_w = reinterpret_cast<VT*>(s_dyn + carve(nrows * RB));
     int32_t* const s_sl = reinterpret_cast<int32_t*>(s_dyn + carve(4 * (part.nslices + 1)));
+    // the rows to push (GRID: the halo rows to poll)
     uint32_t* const s_push = reinterpret_cast<uint32_t*>(s_dyn + carve(4 * part.npush));
     const int o_diag = a.diag ? carve(nrows * RB) : -1;
     const int o_col = carve(2 * part.entries);
     const uint16_t* const g_col = a.loc_col + part.entry_off;
     for (int i = tid; i <= part.nslices; i += CC_T) s_sl[i] = a.slices[part.slice_off + i];
-    for (int i = tid; i < part.npush; i += CC_T) s_push[i] = a.push[part.push_off + i];
+    for (int i = tid; i < part.npush; i += CC_T)
+      s_push[i] = GRID ? (uint32_t)a.halo[part.push_off + i] : a.push[part.push_off + i];
     if (o_col >= 0)
       for (int i = tid; i < part.entries / 8; i += CC_T)
         reinterpret_cast<uint4*>(s_dyn + o_col)[i] = reinterpret_cast<const uint4*>(g_col)[i];
@@ -511,7 +613,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
             }
           }
         }
-        cl_sync();
+        x_sync();
         // a slice at a time: 8 lanes walk a row (coalesced index and value loads, 4 rows per
         // step, the steps' loads in flight together), the sums go to the rows' own lanes
         double rr[NC], bb[NC];
@@ -606,6 +708,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
               acc[s] += (double)r[i][s] * (double)uv[s];
             }
             sts_row<VT, LD>(s_win, lr, uv);
+            publish(row0 + lr, uv);
           }
         }
       } else {
@@ -634,40 +737,85 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
               acc[NC + s] += (double)r[i][s] * (double)r[i][s];
             }
             sts_row<VT, LD>(s_win, lr, uv);
+            publish(row0 + lr, uv);
           }
         }
       }
       // ---- the rows other CTAs hold as halo, then (while they travel) this warp's r.u, r.r
       __syncthreads();
-      if (tid == 0) mb_expect(&s_mb[2], (uint32_t)(part.nhalo * RB) + a.wait_missing);
-      for (int i = tid; i < part.npush; i += CC_T) {
-        const uint32_t e = s_push[i];
-        const uint32_t src = e & ((1u << CC_SRC_BITS) - 1);
-        const uint32_t slot = (e >> CC_SRC_BITS) & ((1u << CC_SLOT_BITS) - 1);
-        const uint32_t dst = e >> (CC_SRC_BITS + CC_SLOT_BITS);
-        cl_send_row<RB>(cl_map(s_win + (size_t)slot * LD, dst), s_win + (size_t)src * LD,
-                        cl_map(&s_mb[2], dst));
+      if constexpr (!GRID) {
+        if (tid == 0) mb_expect(&s_mb[2], (uint32_t)(part.nhalo * RB) + a.wait_missing);
+        for (int i = tid; i < part.npush; i += CC_T) {
+          const uint32_t e = s_push[i];
+          const uint32_t src = e & ((1u << CC_SRC_BITS) - 1);
+          const uint32_t slot = (e >> CC_SRC_BITS) & ((1u << CC_SLOT_BITS) - 1);
+          const uint32_t dst = e >> (CC_SRC_BITS + CC_SLOT_BITS);
+          cl_send_row<RB>(cl_map(s_win + (size_t)slot * LD, dst), s_win + (size_t)src * LD,
+                          cl_map(&s_mb[2], dst));
+        }
       }
       {
         const double v = WarpReduce<2 * NC>::run(acc, lane);
         const int id = WarpReduce<2 * NC>::value_of(lane);
         if (id >= 0) s_red[warp][(id / NC) * 4 + id % NC] = v;
       }
-      // a wait that runs out is acted on after the next CTA barrier, by every thread
-      if (!mb_wait(&s_mb[2], ph_halo, a.wait_limit_ns)) s_gave_up = 1;
-      ph_halo ^= 1u;
+      // a wait that runs out is acted on after a CTA barrier, by every thread
+      if constexpr (GRID) {
+        const uint32_t want = epoch + a.wait_missing;
+        constexpr int U = UW == 1 ? 8 : (UW == 2 ? 4 : 2);
+        for (int i0 = tid; i0 < part.nhalo; i0 += U * CC_T) {
+          ulonglong2 v[U][UW];
+          const ulonglong2* src[U];
+#pragma unroll
+          for (int k = 0; k < U; k++) {
+            const int i = min(i0 + k * CC_T, part.nhalo - 1);
+            src[k] = a.ubuf + (int64_t)s_push[i] * UW;
+#pragma unroll
+            for (int j = 0; j < UW; j++) v[k][j] = ld_unit(src[k] + j);
+          }
+#pragma unroll
+          for (int k = 0; k < U; k++) {
+            if (i0 + k * CC_T < part.nhalo) {
+              VT uv[LD];
+#pragma unroll
+              for (int s = 0; s < LD; s++) uv[s] = VT(0);
+#pragma unroll
+              for (int j = 0; j < UW; j++) {
+                if (!poll_unit<TAG>(src[k] + j, v[k][j], want, a.wait_limit_ns, &s_gave_up))
+                  s_gave_up = 1;
+                if constexpr (sizeof(VT) == 8) {
+                  uv[j] = __longlong_as_double((long long)v[k][j].x);
+                } else {
+                  const uint32_t w[3] = {(uint32_t)v[k][j].x, (uint32_t)(v[k][j].x >> 32),
+                                         (uint32_t)v[k][j].y};
+#pragma unroll
+                  for (int s = 0; s < 3; s++)
+                    if (3 * j + s < LD) uv[3 * j + s] = __uint_as_float(w[s]);
+                }
+              }
+              sts_row<VT, LD>(s_win, nrows + i0 + k * CC_T, uv);
+            }
+          }
+        }
+        __syncthreads();
+      } else {
+        if (!mb_wait(&s_mb[2], ph_halo, a.wait_limit_ns)) s_gave_up = 1;
+        ph_halo ^= 1u;
+      }
 
       // ---- w = A u from the window; w.u
       double wu[NC];
 #pragma unroll
       for (int s = 0; s < NC; s++) wu[s] = 0.0;
+      // columns are byte offsets into the window (GRID: its entries)
+      constexpr uint32_t CU = GRID ? RB : 1;
       const unsigned char* const s_winb = reinterpret_cast<const unsigned char*>(s_win);
       auto gather4 = [&](uint2 c, const VT* v, VT ak[LD], VT ak2[LD]) {
         VT u0[LD], u1[LD], u2[LD], u3[LD];
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x & 0xffffu)), 0, u0);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x >> 16)), 0, u1);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y & 0xffffu)), 0, u2);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y >> 16)), 0, u3);
+        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x & 0xffffu) * CU), 0, u0);
+        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x >> 16) * CU), 0, u1);
+        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y & 0xffffu) * CU), 0, u2);
+        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y >> 16) * CU), 0, u3);
         axpy_row<VT, LD>(v[0], u0, ak);
         axpy_row<VT, LD>(v[1], u1, ak2);
         axpy_row<VT, LD>(v[2], u2, ak);
@@ -781,24 +929,71 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         const int id = WarpReduce<NC>::value_of(lane);
         if (id >= 0) s_red[warp][8 + id] = v;
         __syncthreads();
+        // a CTA that gave up sends no sums, so no other completes this pass either
+        if (s_gave_up) {
+          alive = false;
+          break;
+        }
         const int slot = tid & 15;
         const uint32_t dst = (uint32_t)(tid >> 4);
-        if (dst < C && (slot & 3) < NC && (slot < 12 || first)) {
+        const bool used = (slot & 3) < NC && (slot < 12 || first);
+        if (GRID ? (dst == 0 && used) : (dst < C && used)) {
           double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
           for (int g = 0; g < CC_W; g++) t[g & 3] += s_red[g][slot];
-          cl_send(cl_map(s_part + (buf * 16 + rank) * 16 + slot, dst),
-                  (t[0] + t[1]) + (t[2] + t[3]), cl_map(&s_mb[buf], dst));
+          const double v = (t[0] + t[1]) + (t[2] + t[3]);
+          if constexpr (GRID)
+            st_unit(a.sums + ((int64_t)buf * C + rank) * 16 + slot,
+                    (unsigned long long)__double_as_longlong(v), epoch);
+          else
+            cl_send(cl_map(s_part + (buf * 16 + rank) * 16 + slot, dst), v,
+                    cl_map(&s_mb[buf], dst));
         }
-        if (tid == 0)
-          mb_expect(&s_mb[buf], C * (uint32_t)((first ? 4 : 3) * NC * sizeof(double)) +
-                                    a.wait_missing);
+        if constexpr (!GRID) {
+          if (tid == 0)
+            mb_expect(&s_mb[buf], C * (uint32_t)((first ? 4 : 3) * NC * sizeof(double)) +
+                                      a.wait_missing);
+        } else {
+          // group g of 32 adds the sums of CTAs g, g + 32, ... (up to 5 loads in flight)
+          const int g = tid >> 4;
+          double t2 = 0.0;
+          if (used) {
+            const ulonglong2* src = a.sums + ((int64_t)buf * C + g) * 16 + slot;
+            for (int b0 = g; b0 < (int)C; b0 += 5 * 32, src += 5 * 32 * 16) {
+              ulonglong2 u[5];
+#pragma unroll
+              for (int k = 0; k < 5; k++)
+                if (b0 + 32 * k < (int)C) u[k] = ld_unit(src + 32 * 16 * k);
+#pragma unroll
+              for (int k = 0; k < 5; k++) {
+                if (b0 + 32 * k < (int)C) {
+                  if (!poll_unit<0>(src + 32 * 16 * k, u[k], epoch, a.wait_limit_ns, &s_gave_up))
+                    s_gave_up = 1;
+                  t2 += __longlong_as_double((long long)u[k].x);
+                }
+              }
+            }
+          }
+          s_part[tid] = t2;
+          __syncthreads();
+        }
       }
       // ---- warp 0: totals (lanes l and l + 16 sum half of the CTAs each), lane decisions
       if (warp == 0) {
-        if (!mb_wait(&s_mb[buf], (ph_part >> buf) & 1u, a.wait_limit_ns)) s_gave_up = 1;
+        if constexpr (!GRID)
+          if (!mb_wait(&s_mb[buf], (ph_part >> buf) & 1u, a.wait_limit_ns)) s_gave_up = 1;
         double tot;
-        {
+        if constexpr (GRID) {
+          const double* pp = s_part + (lane & 15) + (lane >> 4) * 16 * 16;
+          double t[16];
+#pragma unroll
+          for (int g = 0; g < 16; g++) t[g] = pp[g * 16];
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int g = 0; g < o; g++) t[g] += t[g + o];
+          tot = t[0] + __shfl_xor_sync(0xffffffffu, t[0], 16);
+        } else {
           const double* pp = s_part + buf * 256 + (lane & 15) + ((lane >> 4) ? 8 * 16 : 0);
           const int nc = (lane >> 4) ? (int)C - 8 : min((int)C, 8);
           double t[8];
@@ -936,6 +1131,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       }
       ph_part ^= 1u << buf;
       buf ^= 1u;
+      epoch++;
       __syncthreads();
       if (s_gave_up) {
         alive = false;
@@ -967,9 +1163,12 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       }
     }
   }
-  // nothing is in flight towards a CTA that finished its solves; after a wait that ran out
-  // the others' sends may be: no CTA leaves before all have given up
-  cl_sync();
+  // nothing is in flight towards a CTA that finished its solve; after a wait that ran out
+  // the others' sends may be: no CTA of a cluster leaves before all have given up
+  if constexpr (GRID)
+    __syncthreads();
+  else
+    cl_sync();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_taddr));
 }
@@ -1008,8 +1207,9 @@ __global__ void k_ccg_slices(CcgPart* parts, const int32_t* __restrict__ indptr,
 // One block per part.  The halo as a bitmap over the system's rows (shared memory), so its
 // ascending order and every column's window slot come from popcounts.  FILL = false: the
 // halo size and, per rank, the halo positions where that rank's rows begin; window-local
-// columns.  FILL = true: the push entries (rank of this part, slot, source row) into the
-// producers' lists at push_at (per producer and consumer).
+// columns (times rb).  FILL = true: the push entries (rank of this part, slot, source row)
+// into the producers' lists at push_at (per producer and consumer), or, when halo is given
+// (GRID), the halo's rows at the part's push_off.
 template <bool FILL>
 __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sys_row0,
                            const int32_t* __restrict__ sys_rows,
@@ -1018,7 +1218,8 @@ __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sy
                            const int32_t* __restrict__ slices, int rb,
                            uint16_t* __restrict__ loc_col,
                            int32_t* __restrict__ bounds, const int32_t* __restrict__ push_at,
-                           uint32_t* __restrict__ push, int32_t* __restrict__ flag) {
+                           uint32_t* __restrict__ push, int32_t* __restrict__ halo,
+                           int32_t* __restrict__ flag) {
   extern __shared__ uint32_t s_bits[];
   const int sys = blockIdx.x / C, rank = blockIdx.x % C;
   const CcgPart p = parts[blockIdx.x];
@@ -1068,7 +1269,7 @@ __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sy
   };
   const CcgPart* sp = parts + (int64_t)sys * C;
   if constexpr (!FILL) {
-    for (int k = threadIdx.x; k <= C; k += blockDim.x) {
+    for (int k = threadIdx.x; bounds && k <= C; k += blockDim.x) {
       // halo entries with a row below rank k's first row (ranks in row order)
       const int j = (k < C) ? min(sp[k].row0 - base, n) : n;
       bounds[(int64_t)blockIdx.x * (C + 1) + k] = (j < n) ? halo_pos(j) : s_tot[W];
@@ -1099,6 +1300,10 @@ __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sy
       while (m) {
         const int j = 32 * i + __ffs(m) - 1;
         m &= m - 1;
+        if (halo) {
+          halo[p.push_off + halo_pos(j)] = base + j;
+          continue;
+        }
         int lo = 0, hi = C;  // the last rank whose first row is <= j owns it
         while (hi - lo > 1) {
           const int mid = (lo + hi) >> 1;
@@ -1132,11 +1337,16 @@ struct CcgClass {
   uint16_t* d_cols = nullptr;
   uint32_t* d_push = nullptr;
   void* d_packed = nullptr;
+  // all SMs on one system: halo rows; barrier, sums and published rows (cleared per solve)
+  bool grid = false;
+  int32_t* d_halo = nullptr;
+  char* d_xch = nullptr;
+  size_t xch_bytes = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   ~CcgClass() {
     for (void* p : {(void*)d_parts, (void*)d_order, (void*)d_slices, (void*)d_cols, (void*)d_push,
-                    d_packed})
+                    d_packed, (void*)d_halo, (void*)d_xch})
       if (p) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
     if (done) cudaEventDestroy(done);
@@ -1159,24 +1369,39 @@ namespace {
 
 // The largest rows per thread whose five register vectors fit beside the product (about
 // 60 of 128 registers), and a small form for systems of few rows.
-template <typename VT, int NC>
+template <typename VT, int NC, bool GRID>
 struct Rpt {
   static constexpr int words = NC * (int)sizeof(VT) / 4;
-  static constexpr int big = words == 1 ? 9 : (words == 2 ? 6 : (words <= 4 ? 3 : 2));
-  static constexpr int small = words <= 2 ? 2 : 1;
+  static constexpr int big = words == 1   ? 9
+                             : words == 2 ? 6
+                             : words == 3 ? (GRID ? 4 : 3)
+                             : words == 4 ? 3
+                                          : 2;
+  static constexpr int small = GRID ? (words <= 2 ? 4 : (words <= 4 ? 2 : 1)) : (words <= 2 ? 2 : 1);
 };
 
-template <typename VT, int LD, int NC>
+template <typename VT, int LD, int NC, bool GRID>
 void* pick(int rpt, int* big) {
-  *big = Rpt<VT, NC>::big;
-  return rpt <= Rpt<VT, NC>::small ? (void*)k_ccg<VT, LD, NC, Rpt<VT, NC>::small>
-                                   : (void*)k_ccg<VT, LD, NC, Rpt<VT, NC>::big>;
+  using R = Rpt<VT, NC, GRID>;
+  *big = R::big;
+  return rpt <= R::small ? (void*)k_ccg<VT, LD, NC, R::small, GRID>
+                         : (void*)k_ccg<VT, LD, NC, R::big, GRID>;
 }
-template <typename VT>
+template <typename VT, bool GRID>
 void* pick_ld(int ld, int S, int rpt, int* big) {
-  if (ld == 1) return pick<VT, 1, 1>(rpt, big);
-  if (ld == 2) return pick<VT, 2, 2>(rpt, big);
-  return S <= 3 ? pick<VT, 4, 3>(rpt, big) : pick<VT, 4, 4>(rpt, big);
+  if (ld == 1) return pick<VT, 1, 1, GRID>(rpt, big);
+  if (ld == 2) return pick<VT, 2, 2, GRID>(rpt, big);
+  return S <= 3 ? pick<VT, 4, 3, GRID>(rpt, big) : pick<VT, 4, 4, GRID>(rpt, big);
+}
+void* pick_kernel(bool fp32, bool grid, int ld, int S, int rpt, int* big) {
+  if (grid)
+    return fp32 ? pick_ld<float, true>(ld, S, rpt, big) : pick_ld<double, true>(ld, S, rpt, big);
+  return fp32 ? pick_ld<float, false>(ld, S, rpt, big) : pick_ld<double, false>(ld, S, rpt, big);
+}
+// 16-byte units of a published row
+int row_units(bool fp32, int ld, int S) {
+  const int nc = ld == 1 ? 1 : (ld == 2 ? 2 : (S <= 3 ? 3 : 4));
+  return fp32 ? (nc + 2) / 3 : nc;
 }
 
 template <typename T>
@@ -1207,6 +1432,10 @@ void fill(CcgArgs<VT>& a, const CcgClass* h, const CreateArgs& ca, int win_cap) 
   a.slices = h->d_slices;
   a.loc_col = h->d_cols;
   a.push = h->d_push;
+  a.halo = h->d_halo;
+  a.bar = reinterpret_cast<unsigned int*>(h->d_xch);
+  a.sums = reinterpret_cast<ulonglong2*>(h->d_xch + 256);
+  a.ubuf = a.sums + (size_t)2 * 16 * h->C;
   a.packed = static_cast<VT*>(h->d_packed);
   a.inK = sizeof(VT) == 4 ? (const VT*)op->K32 : (const VT*)op->K64;
   a.sK = static_cast<const VT*>(ca.src->sK);
@@ -1253,11 +1482,11 @@ cudaLaunchConfig_t launch_config(const CcgClass* c, cudaLaunchAttribute* attr, i
   return cfg;
 }
 
-// Tables of the systems `sys` (largest first) on clusters of C CTAs; *ok = false when one
-// does not fit.
+// Tables of the systems `sys` (largest first) on clusters of C CTAs (grid: one system on C
+// CTAs of the whole device); *ok = false when one does not fit.
 int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::vector<int32_t>& sys,
                 const std::vector<int32_t>& row0, const std::vector<int32_t>& rows, int C,
-                bool* ok) {
+                bool grid, bool* ok) {
   *ok = false;
   const tp_csr_op* op = ca.op;
   cudaStream_t st = ca.st;
@@ -1268,8 +1497,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   TP_CUDA_TRY(cudaGetDevice(&dev));
   TP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int rpt = rows_per_thread(most, C);
-  void* fn = inner_fp32 ? pick_ld<float>(ld, op->S, rpt, &big)
-                        : pick_ld<double>(ld, op->S, rpt, &big);
+  void* fn = pick_kernel(inner_fp32 != 0, grid, ld, op->S, rpt, &big);
   if (rpt > big || rpt * CC_T > (1 << CC_SRC_BITS)) return TP_OK;
   cudaFuncAttributes fa;
   TP_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
@@ -1279,6 +1507,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   h->nsys = nsys;
   h->dyn = dyn;
   h->fn = fn;
+  h->grid = grid;
   const int np = nsys * C;
   std::vector<CcgPart> parts(np);
   std::vector<int32_t> base(nsys), count(nsys);
@@ -1324,7 +1553,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
       if (p) cudaFree(p);
     }
   } tmp;
-  const size_t n_bounds = (size_t)np * (C + 1), n_at = (size_t)np * C;
+  const size_t n_bounds = grid ? 0 : (size_t)np * (C + 1), n_at = grid ? 0 : (size_t)np * C;
   TP_CUDA_TRY(dev_alloc(&tmp.p, 2 * (size_t)nsys + n_bounds + n_at + 1));
   int32_t *t_row0 = tmp.p, *t_rows = tmp.p + nsys, *t_bounds = tmp.p + 2 * (size_t)nsys,
           *t_at = t_bounds + n_bounds, *t_flag = t_at + n_at;
@@ -1337,16 +1566,25 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
                               cudaMemcpyHostToDevice, st));
   TP_CUDA_TRY(cudaMemsetAsync(t_flag, 0, sizeof(int32_t), st));
   const size_t bits = 2 * sizeof(uint32_t) * (size_t)((most + 31) / 32);
-  if (bits > 40 * 1024) return TP_OK;
+  if (bits > 200 * 1024) return TP_OK;
+  if (bits > 40 * 1024) {
+    TP_CUDA_TRY(cudaFuncSetAttribute(k_ccg_halo<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     200 * 1024));
+    TP_CUDA_TRY(cudaFuncSetAttribute(k_ccg_halo<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     200 * 1024));
+  }
+  const int unit = grid ? 1 : (int)rb;  // columns: window entries, or byte offsets
   k_ccg_halo<false><<<np, 512, bits, st>>>(h->d_parts, C, t_row0, t_rows, op->indptr,
-                                           op->indices, h->d_slices, (int)rb, h->d_cols,
-                                           t_bounds, nullptr, nullptr, t_flag);
+                                           op->indices, h->d_slices, unit, h->d_cols,
+                                           grid ? nullptr : t_bounds, nullptr, nullptr, nullptr,
+                                           t_flag);
   TP_LAUNCH_CHECK();
   std::vector<int32_t> bounds(n_bounds), at(n_at);
   int32_t flag = 0;
   TP_CUDA_TRY(cudaMemcpyAsync(parts.data(), h->d_parts, sizeof(CcgPart) * np,
                               cudaMemcpyDeviceToHost, st));
-  TP_CUDA_TRY(cudaMemcpyAsync(bounds.data(), t_bounds, sizeof(int32_t) * n_bounds,
+  if (!grid)
+    TP_CUDA_TRY(cudaMemcpyAsync(bounds.data(), t_bounds, sizeof(int32_t) * n_bounds,
                               cudaMemcpyDeviceToHost, st));
   TP_CUDA_TRY(cudaMemcpyAsync(&flag, t_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   TP_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1358,7 +1596,8 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
     for (int k = 0; k < C; k++) {
       CcgPart& p = parts[(size_t)q * C + k];
       p.push_off = (int32_t)npush;
-      for (int j = 0; j < C; j++) {
+      if (grid) npush += p.nhalo;
+      for (int j = 0; j < C && !grid; j++) {
         at[((size_t)q * C + k) * C + j] = (int32_t)npush;
         const int32_t* bj = &bounds[((size_t)q * C + j) * (C + 1)];
         // empty ranks past the last row share its bound: they own nothing
@@ -1368,8 +1607,9 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
       win_cap = std::max(win_cap, p.nrows + p.nhalo);
     }
   win_cap = (win_cap + 3) & ~3;
-  // window columns are 16-bit byte offsets
-  if (npush > INT32_MAX || win_cap >= (1 << CC_SLOT_BITS) || rb * win_cap > 65536) return TP_OK;
+  // window columns are 16-bit
+  if (npush > INT32_MAX || win_cap * unit > 65536) return TP_OK;
+  if (!grid && win_cap >= (1 << CC_SLOT_BITS)) return TP_OK;
   // what has to fit in shared memory (the kernel carves in the same order); columns and
   // values stream from L2 where they do not
   bool spill = false;
@@ -1383,28 +1623,39 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
     need += r16(2 * (size_t)p.entries) + r16(vt * nval);
     spill |= nval > 0 && need > dyn;
   }
-  TP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   if ((int)dyn > fa.maxDynamicSharedSizeBytes)
     TP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = launch_config(h, &attr, 1, st);
-  int active = 0;
-  if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) {
-    cudaGetLastError();
-    return TP_OK;
+  if (grid) {
+    int occ = 0;
+    TP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, CC_T, dyn));
+    if (occ < 1) return TP_OK;
+    TP_CUDA_TRY(dev_alloc(&h->d_halo, (size_t)npush));
+    h->xch_bytes = 256 + sizeof(ulonglong2) * ((size_t)2 * 16 * C +
+                                               (size_t)most * row_units(inner_fp32 != 0, ld, op->S));
+    TP_CUDA_TRY(dev_alloc(&h->d_xch, h->xch_bytes));
+  } else {
+    TP_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = launch_config(h, &attr, 1, st);
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) {
+      cudaGetLastError();
+      return TP_OK;
+    }
   }
-  TP_CUDA_TRY(dev_alloc(&h->d_push, (size_t)npush));
+  if (!grid) TP_CUDA_TRY(dev_alloc(&h->d_push, (size_t)npush));
   TP_CUDA_TRY(dev_alloc(&h->d_order, (size_t)nsys));
   if (spill) TP_CUDA_TRY(cudaMalloc(&h->d_packed, vt * std::max<size_t>((size_t)entries, 1)));
   TP_CUDA_TRY(cudaMemcpyAsync(h->d_order, sys.data(), sizeof(int32_t) * nsys,
                               cudaMemcpyHostToDevice, st));
   TP_CUDA_TRY(cudaMemcpyAsync(h->d_parts, parts.data(), sizeof(CcgPart) * np,
                               cudaMemcpyHostToDevice, st));
-  TP_CUDA_TRY(cudaMemcpyAsync(t_at, at.data(), sizeof(int32_t) * n_at, cudaMemcpyHostToDevice,
-                              st));
+  if (!grid)
+    TP_CUDA_TRY(cudaMemcpyAsync(t_at, at.data(), sizeof(int32_t) * n_at, cudaMemcpyHostToDevice,
+                                st));
   k_ccg_halo<true><<<np, 512, bits, st>>>(h->d_parts, C, t_row0, t_rows, op->indptr,
-                                          op->indices, h->d_slices, (int)rb, h->d_cols, t_bounds,
-                                          t_at, h->d_push, t_flag);
+                                          op->indices, h->d_slices, unit, h->d_cols, t_bounds,
+                                          t_at, h->d_push, grid ? h->d_halo : nullptr, t_flag);
   TP_LAUNCH_CHECK();
   TP_CUDA_TRY(cudaStreamSynchronize(st));
   if (h->fp32)
@@ -1418,8 +1669,8 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
 }  // namespace
 
 int ccg_create(const tp_csr_op* op, int inner_fp32, const CcgSource& src, int max_it,
-               double delta, const double* b, double* x, const double* rtol, cudaStream_t st,
-               Ccg** out) {
+               double delta, const double* b, double* x, const double* rtol, bool allow_grid,
+               cudaStream_t st, Ccg** out) {
   *out = nullptr;
   if (op->M64 || op->n_rows <= 0) return TP_OK;
   const int nsys = op->n_systems > 0 ? op->n_systems : 1;
@@ -1437,18 +1688,19 @@ int ccg_create(const tp_csr_op* op, int inner_fp32, const CcgSource& src, int ma
     most = std::max(most, r1 - r0);
   }
   int big = 0;
-  if (inner_fp32)
-    pick_ld<float>(op->ld, op->S, 1, &big);
-  else
-    pick_ld<double>(op->ld, op->S, 1, &big);
-  // One system: up to where one cluster beats the grid engine (us per iteration, cluster /
-  // grid): one FP64 column 2.2 / 7.5 at 4.9k rows, 6.3 / 7.9 at 39k, 8.4 / 8.1 at 47k; two
-  // FP32 columns 3.5 / 6.3 at 14k, 8.7 / 6.4 at 43k (equal near 29k); one FP32 column 6.3 /
-  // 8.2 at 69k and three 5.5 / 6.5 at 24k, both at the register limit.
-  int most_rpt = big;
-  if (nsys == 1 && !inner_fp32 && op->ld == 1) most_rpt = 5;
-  if (nsys == 1 && inner_fp32 && op->ld == 2) most_rpt = 3;
-  if (rows_per_thread(most, 16) > most_rpt) return TP_OK;
+  pick_kernel(inner_fp32 != 0, false, op->ld, op->S, 1, &big);
+  // One system: a cluster up to where every SM is faster (us per iteration, cluster / all
+  // SMs): one FP64 column 3.1 / 4.0 at 15.6k rows, 4.3 / 4.2 at 24k, 6.3 / 4.4 at 39k; two
+  // 3.9 / 4.0 at 9.3k; three 5.0 / 4.3 and four 5.0 / 5.1 at 4.9k; one FP32 column 4.0 / 4.4
+  // at 36k, 4.9 / 4.4 at 51k; two 3.5 / 4.1 and three 4.1 / 4.3 at 13.8k, 5.6 / 4.1 and
+  // 5.5 / 4.4 at 24k; four 4.6 / 4.5 at 9.3k.
+  bool grid = rows_per_thread(most, 16) > big;
+  if (allow_grid && nsys == 1) {
+    const int64_t limit = inner_fp32 ? (op->ld == 1 ? 40960 : (op->S <= 3 ? 16384 : 8192))
+                                     : (op->ld == 1 ? 24576 : (op->ld == 2 ? 8192 : 4096));
+    grid = grid || most > limit;
+  }
+  if (grid && !(allow_grid && nsys == 1)) return TP_OK;
   std::stable_sort(order.begin(), order.end(),
                    [&](int32_t p, int32_t q) { return rows[p] > rows[q]; });
   Ccg* h = new Ccg();
@@ -1467,14 +1719,14 @@ int ccg_create(const tp_csr_op* op, int inner_fp32, const CcgSource& src, int ma
   const int least = nsys > 8 ? 8 : 16;
   auto fits8 = [&](int32_t m) { return least == 8 && rows_per_thread(rows[m], 8) <= big; };
   for (int at = 0; at < nsys;) {
-    const int C = fits8(order[at]) ? 8 : 16;
+    const int C = grid ? sm_count() : (fits8(order[at]) ? 8 : 16);
     int end = at + 1;
     while (end < nsys && (C == least || !fits8(order[end]))) end++;
     const std::vector<int32_t> sys(order.begin() + at, order.begin() + end);
     CcgClass* c = new CcgClass();
     h->classes.push_back(c);
     bool ok = false;
-    const int rc = build_class(c, ca, inner_fp32, sys, row0, rows, C, &ok);
+    const int rc = build_class(c, ca, inner_fp32, sys, row0, rows, C, grid, &ok);
     if (rc != TP_OK || !ok) return rc;
     at = end;
   }
@@ -1497,9 +1749,14 @@ int ccg_run(Ccg* h, cudaStream_t st) {
   for (CcgClass* c : h->classes) {
     cudaStream_t s = fork ? c->stream : st;
     if (fork) TP_CUDA_TRY(cudaStreamWaitEvent(s, h->begin, 0));
+    void* args[1] = {c->fp32 ? (void*)&c->af : (void*)&c->ad};
+    if (c->grid) {
+      TP_CUDA_TRY(cudaMemsetAsync(c->d_xch, 0, c->xch_bytes, s));
+      TP_CUDA_TRY(cudaLaunchCooperativeKernel(c->fn, dim3(c->C), dim3(CC_T), args, c->dyn, s));
+      continue;
+    }
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = launch_config(c, &attr, c->nsys, s);
-    void* args[1] = {c->fp32 ? (void*)&c->af : (void*)&c->ad};
     TP_CUDA_TRY(cudaLaunchKernelExC(&cfg, c->fn, args));
     if (fork) {
       TP_CUDA_TRY(cudaEventRecord(c->done, s));
@@ -1538,6 +1795,7 @@ int ccg_result(Ccg* h, tp_cg_result* res, int32_t* lane_iters, int32_t* lane_sta
 }
 
 size_t ccg_smem(const Ccg* h) { return h->classes[0]->dyn; }
+bool ccg_is_grid(const Ccg* h) { return h->classes[0]->grid; }
 
 void ccg_set_wait(Ccg* h, unsigned long long limit_ns, unsigned int missing) {
   for (CcgClass* c : h->classes) {

@@ -1129,8 +1129,8 @@ extern "C" int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const 
   // systems that fit one thread-block cluster each run there; the host-loop variant
   // (use_graph_loop = 0) always is the graph engine
   if (h->use_cond) {
-    rc = ccg_create(op, cfg->inner_fp32, CcgSource{}, cfg->max_it, delta, b, x, rtol, st,
-                    &h->ccg);
+    rc = ccg_create(op, cfg->inner_fp32, CcgSource{}, cfg->max_it, delta, b, x, rtol,
+                    false, st, &h->ccg);
     if (rc) {
       tp_cg_destroy(h);
       return rc;

@@ -3797,7 +3797,7 @@ extern "C" int tp_pcg_create(const tp_csr_op* op, const tp_sell* sell, int max_i
     CcgSource src;
     src.sK = inner_fp32 ? (const void*)sell->sK32 : (const void*)sell->sK64;
     src.slice_ptr = sell->slice_ptr;
-    rc = ccg_create(op, h->fp32, src, max_it, d, b, x, rtol, st, &h->ccg);
+    rc = ccg_create(op, h->fp32, src, max_it, d, b, x, rtol, true, st, &h->ccg);
   }
   if (rc == TP_OK && !h->ccg) {
     rc = try_window(h, sell, hasM, st);
@@ -3868,7 +3868,7 @@ extern "C" int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block) {
 
 extern "C" int tp_pcg_engine(tp_pcg_handle* h, int* window, size_t* smem_bytes) {
   TP_REQUIRE(h, "null handle");
-  if (window) *window = h->ccg ? 4 : h->window;
+  if (window) *window = !h->ccg ? h->window : (ccg_is_grid(h->ccg) ? 5 : 4);
   if (smem_bytes) *smem_bytes = h->dyn_smem;
   if (smem_bytes && h->ccg) *smem_bytes = ccg_smem(h->ccg);
   return TP_OK;

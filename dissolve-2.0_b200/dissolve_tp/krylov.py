@@ -264,11 +264,13 @@ class PersistentCG:
     def engine(self) -> dict:
         """Engine of the handle: shared-memory window (Chronopoulos-Gear; `tmem`: with the
         recurrence vectors in tensor memory; `pipelined`: the one-barrier pipelined form,
-        vectors in tensor memory; `cluster`: one thread-block cluster) or streaming."""
+        vectors in tensor memory; `cluster`: one thread-block cluster; `exchange`: every SM, data exchanged
+        with its pass number and no barrier per iteration) or streaming."""
         w, sm = ctypes.c_int(0), ctypes.c_size_t(0)
         call("tp_pcg_engine", self._h, ctypes.byref(w), ctypes.byref(sm))
         return {"window": bool(w.value), "tmem": w.value in (2, 3), "pipelined": w.value == 3,
-                "cluster": w.value == 4, "smem_bytes": int(sm.value)}
+                "cluster": w.value == 4, "exchange": w.value == 5,
+                "smem_bytes": int(sm.value)}
 
     def run(self):
         call("tp_pcg_run", self._h, stream_handle())

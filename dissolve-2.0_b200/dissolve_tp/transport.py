@@ -162,6 +162,7 @@ class BatchedTransport:
             eng = self.solver.engine()
             self.cg_config["form"] = (
                 "cluster (Chronopoulos-Gear, one thread-block cluster)" if eng["cluster"] else
+                "window (Chronopoulos-Gear, exchange by tagged data)" if eng["exchange"] else
                 "window (pipelined, vectors in tensor memory)" if eng["pipelined"] else
                 "window (Chronopoulos-Gear, vectors in tensor memory)" if eng["tmem"] else
                 "window (Chronopoulos-Gear)" if eng["window"] else "streaming")

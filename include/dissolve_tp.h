@@ -530,9 +530,13 @@ TP_API int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block);
  * the same tensor-memory layout, for at most 3 columns (DISSOLVE_PCG_PIPE=0 at create keeps
  * engine 2); it refreshes at least every factor 1e3 of residual reduction whatever
  * `delta` asks for.  *window = 4: the Chronopoulos-Gear form in one thread-block cluster,
- * for a system that fits one (as for tp_cg_engine; not when the environment names one of
- * the grid engines through a DISSOLVE_PCG_* variable, or ctas_per_sm is given); profiled
- * runs use the grid engine of the handle.
+ * for systems of up to about 41k rows (one FP32 column), 25k (one FP64 column) or 16k (two
+ * or three FP32 columns).  *window = 5: the same passes on every SM for larger systems, the
+ * data exchanged with its pass number and no barrier per iteration (up to 1.3M rows for one
+ * FP32 column, 450k for one FP64 column, 300k for three FP32 columns, while the windows fit
+ * shared memory).  Engines 4 and 5 take no mass matrix, and are not chosen when the
+ * environment names one of the others through a DISSOLVE_PCG_* variable or ctas_per_sm is
+ * given; profiled runs use the grid engine of the handle.
  * *window = 0: the streaming engine (standard recurrences, columns and
  * gathers from global memory).  *smem_bytes: dynamic shared memory per CTA.  The
  * environment variable DISSOLVE_PCG_ENGINE=stream at create forces the streaming

@@ -1,7 +1,7 @@
-"""The cluster engine (one thread-block cluster per system) against the grid and graph
-engines and the FP64 oracle: every element type and column count, Dirichlet rows, systems
-whose row ranges leave ranks of the cluster empty or partly filled, the largest systems
-that fit (columns and values streamed from L2) and the queue of many systems.
+"""The cluster engine (one thread-block cluster per system) and the exchange engine (the
+same passes on every SM) against the grid and graph engines: every element type and column
+count, Dirichlet rows, systems whose row ranges leave CTAs empty or partly filled, both
+sides of the size where one engine hands over to the other, and many systems at once.
 
 Bars: each solve converges on its FP64 residual (||b - A x|| <= rtol ||b||); solutions of
 two engines at rtol 1e-11 agree within 1e-8 relative L2 (the residual rule times the
@@ -48,12 +48,19 @@ def _check(op, sol, res, b, rtol):
     assert np.all(np.abs(rn - res["rnorm"]) <= 0.01 * res["rnorm"] + 1e-14 * res["bnorm"])
 
 
-@pytest.mark.parametrize("n,S,fp32,bc", [
-    (1, 1, False, False), (3, 1, True, False), (7, 2, False, True), (9, 3, True, True),
-    (12, 4, True, False), (10, 4, False, False), (16, 1, False, True), (20, 2, True, False),
-    (23, 3, True, False), (27, 4, True, False), (28, 2, False, False), (24, 3, False, False),
-    (33, 1, False, False), (35, 1, False, False), (40, 1, True, False)])
-def test_cluster_matches_grid_engine(cuda_device, monkeypatch, n, S, fp32, bc):
+@pytest.mark.parametrize("n,S,fp32,bc,engine", [
+    (1, 1, False, False, "cluster"), (3, 1, True, False, "cluster"),
+    (7, 2, False, True, "cluster"), (9, 3, True, True, "cluster"),
+    (12, 4, True, False, "cluster"), (10, 4, False, False, "cluster"),
+    (16, 1, False, True, "cluster"), (20, 2, True, False, "cluster"),
+    (23, 3, True, False, "cluster"), (28, 1, False, False, "cluster"),
+    (33, 1, True, False, "cluster"), (29, 1, False, True, "exchange"),
+    (35, 1, True, True, "exchange"), (26, 3, True, True, "exchange"),
+    (27, 4, True, False, "exchange"), (28, 2, False, False, "exchange"),
+    (24, 3, False, False, "exchange"), (22, 4, False, True, "exchange"),
+    (34, 2, True, False, "exchange"), (48, 1, False, False, "exchange"),
+    (44, 3, True, False, "exchange")])
+def test_engine_matches_grid_engine(cuda_device, monkeypatch, n, S, fp32, bc, engine):
     import torch
     from dissolve_tp.krylov import PersistentCG
     asm, op, b = _operator(n, S, fp32, bc)
@@ -61,9 +68,8 @@ def test_cluster_matches_grid_engine(cuda_device, monkeypatch, n, S, fp32, bc):
     one = PersistentCG(op, **kw)
     monkeypatch.setenv("DISSOLVE_PCG_PIPE", "0")
     grid = PersistentCG(op, **kw)
-    assert not grid.engine()["cluster"]
-    fits = one.engine()["cluster"]
-    assert fits == ((n, S, fp32) not in ((24, 3, False), (35, 1, False)))  # past the limits
+    assert one.engine()[engine], one.engine()
+    assert not grid.engine()["cluster"] and not grid.engine()["exchange"]
     out = []
     for sol in (one, grid):
         sol.b.copy_(b)
@@ -127,6 +133,53 @@ def test_cluster_solve_is_captured_in_a_graph(cuda_device):
     sol = PersistentCG(op, rtol=1e-10, max_it=2000, inner_fp32=True)
     sol.b.copy_(b)
     sol.x.zero_()
+    ref = sol.solve()
+    x = sol.x.clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        sol.run()
+    for _ in range(2):
+        sol.x.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(sol.x, x) and sol.result()["iterations"] == ref["iterations"]
+
+
+@pytest.mark.parametrize("n,S,fp32", [(30, 1, False), (26, 3, True)])
+def test_exchange_wait_runs_out_then_recovers(cuda_device, n, S, fp32):
+    """Every wait expects a pass number that never comes: the solve ends with TP_ERR_TIMEOUT
+    after the 1 ms limit and the handle then solves with the same bits as before."""
+    import time
+
+    import torch
+    from dissolve_tp.krylov import PersistentCG
+    asm, op, b = _operator(n, S, fp32, False)
+    sol = PersistentCG(op, rtol=1e-10, max_it=4000, inner_fp32=fp32)
+    assert sol.engine()["exchange"]
+    sol.b.copy_(b)
+    ref = sol.solve()
+    x = sol.x.clone()
+    assert ref["converged"]
+    sol.set_wait_limit(1e-3, missing_arrivals=1)
+    sol.x.zero_()
+    t0 = time.perf_counter()
+    res = sol.solve()
+    assert res["status"] == 9 and list(res["lane_status"]) == [9] * S
+    assert time.perf_counter() - t0 < 1.0
+    sol.set_wait_limit(0.0, 0)
+    sol.x.zero_()
+    res = sol.solve()
+    assert res["converged"] and res["iterations"] == ref["iterations"]
+    assert torch.equal(sol.x, x)
+
+
+def test_exchange_solve_is_captured_in_a_graph(cuda_device):
+    import torch
+    from dissolve_tp.krylov import PersistentCG
+    asm, op, b = _operator(28, 3, True, True)
+    sol = PersistentCG(op, rtol=1e-10, max_it=2000, inner_fp32=True)
+    assert sol.engine()["exchange"]
+    sol.b.copy_(b)
     ref = sol.solve()
     x = sol.x.clone()
     g = torch.cuda.CUDAGraph()
