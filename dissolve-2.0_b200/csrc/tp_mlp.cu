@@ -121,91 +121,79 @@ struct MlpSmem {
   float b3;
 };
 
-// W2T (optional, the backward pass): W2 transposed, [in][out]
+// W2T (the backward pass): W2 transposed, [in][out]
 __device__ void load_weights(MlpSmem& sm, const float* __restrict__ P,
-                             __nv_bfloat16 (*W2T)[W2S] = nullptr) {
-  for (int i = threadIdx.x; i < MLP_H * MLP_IN; i += blockDim.x)
-    sm.W1[i / MLP_IN][i % MLP_IN] = __float2bfloat16_rn(P[OFF_W1 + i]);
-  for (int i = threadIdx.x; i < MLP_H * MLP_H; i += blockDim.x) {
-    const __nv_bfloat16 w = __float2bfloat16_rn(P[OFF_W2 + i]);
-    sm.W2[i / MLP_H][i % MLP_H] = w;
-    if (W2T) W2T[i % MLP_H][i / MLP_H] = w;
-  }
-  for (int i = threadIdx.x; i < MLP_H; i += blockDim.x) {
+                             __nv_bfloat16 (*W2T)[W2S]) {
+  // every load of a thread in flight before its first conversion
+  constexpr int T = 128, N1 = MLP_H * MLP_IN / T, N2 = MLP_H * MLP_H / T;
+  float w1[N1], w2[N2];
+#pragma unroll
+  for (int k = 0; k < N1; k++) w1[k] = __ldg(P + OFF_W1 + k * T + threadIdx.x);
+#pragma unroll
+  for (int k = 0; k < N2; k++) w2[k] = __ldg(P + OFF_W2 + k * T + threadIdx.x);
+  for (int i = threadIdx.x; i < MLP_H; i += T) {
     sm.w3[i] = __bfloat162float(__float2bfloat16_rn(P[OFF_W3 + i]));
     sm.b1[i] = P[OFF_B1 + i];
     sm.b2[i] = P[OFF_B2 + i];
   }
   if (threadIdx.x == 0) sm.b3 = P[OFF_B3];
+#pragma unroll
+  for (int k = 0; k < N1; k++) {
+    const int i = k * T + threadIdx.x;
+    sm.W1[i / MLP_IN][i % MLP_IN] = __float2bfloat16_rn(w1[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < N2; k++) {
+    const int i = k * T + threadIdx.x;
+    const __nv_bfloat16 w = __float2bfloat16_rn(w2[k]);
+    sm.W2[i / MLP_H][i % MLP_H] = w;
+    W2T[i % MLP_H][i / MLP_H] = w;
+  }
   __syncthreads();
 }
 
-// B fragment of W^T for W stored [n][k] row-major with row length ldk
-__device__ __forceinline__ void bfrag(const __nv_bfloat16* W, int ldk, int n0, int k0, int g,
-                                      int t, uint32_t& b0, uint32_t& b1) {
-  const __nv_bfloat16* row = W + (n0 + g) * ldk + k0 + 2 * t;
-  b0 = *reinterpret_cast<const uint32_t*>(row);
-  b1 = *reinterpret_cast<const uint32_t*>(row + 8);
+// four 8x8 matrices of a row-major BF16 array, lane l giving the address of row l % 8 of
+// matrix l / 8: fragments (row g, columns 2t, 2t + 1) into registers ...
+__device__ __forceinline__ void ldm4(uint32_t r[4], const __nv_bfloat16* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a)
+               : "memory");
+}
+// ... and fragments stored transposed (row g of the fragment becomes column g)
+__device__ __forceinline__ void stm4t(__nv_bfloat16* p, const uint32_t r[4]) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(a),
+               "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
 }
 
-// Forward pass of one 16-row tile.  xa: the A fragment of the inputs (K = 16).
-// On return z1/z2 hold the pre-activations (8 n-tiles x 4), y the output of rows g, g+8
-// (valid in every lane of the quad).
-__device__ __forceinline__ void mlp_tile_forward(const MlpSmem& sm, const uint32_t xa[4], int g,
-                                                 int t, float z1[8][4], float z2[8][4],
-                                                 float& y0, float& y1) {
+// C[n-tile n] += A (4 k-steps of fragments) B, B[k][j] = W[j][k] for W [64][ldk] row-major
+__device__ __forceinline__ void mma_64x64(float c[8][4], const uint32_t a[4][4],
+                                          const __nv_bfloat16* W, int ldk, int lane) {
 #pragma unroll
   for (int n = 0; n < 8; n++) {
-    const float bl = sm.b1[n * 8 + 2 * t], bh = sm.b1[n * 8 + 2 * t + 1];
-    z1[n][0] = bl;
-    z1[n][1] = bh;
-    z1[n][2] = bl;
-    z1[n][3] = bh;
-    uint32_t b0, b1;
-    bfrag(&sm.W1[0][0], W1S, n * 8, 0, g, t, b0, b1);
-    mma_bf16(z1[n], xa[0], xa[1], xa[2], xa[3], b0, b1);
+    uint32_t b[8];  // k = 0..31, 32..63 of the tile's 8 columns
+    ldm4(b, W + (n * 8 + (lane & 7)) * ldk + (lane >> 3) * 8);
+    ldm4(b + 4, W + (n * 8 + (lane & 7)) * ldk + 32 + (lane >> 3) * 8);
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++)
+      mma_bf16(c[n], a[kk][0], a[kk][1], a[kk][2], a[kk][3], b[2 * kk], b[2 * kk + 1]);
   }
-  uint32_t ha[4][4];  // h1 as A fragments, 4 k-steps
+}
+
+// BF16 A fragments of max(z, 0) for the 8 n-tiles of a 16 x 64 accumulator
+__device__ __forceinline__ void relu_fragments(const float z[8][4], uint32_t a[4][4]) {
 #pragma unroll
   for (int kk = 0; kk < 4; kk++) {
-    const float* lo = z1[2 * kk];
-    const float* hi = z1[2 * kk + 1];
-    ha[kk][0] = pack_bf16(fmaxf(lo[0], 0.f), fmaxf(lo[1], 0.f));
-    ha[kk][1] = pack_bf16(fmaxf(lo[2], 0.f), fmaxf(lo[3], 0.f));
-    ha[kk][2] = pack_bf16(fmaxf(hi[0], 0.f), fmaxf(hi[1], 0.f));
-    ha[kk][3] = pack_bf16(fmaxf(hi[2], 0.f), fmaxf(hi[3], 0.f));
+    const float* lo = z[2 * kk];
+    const float* hi = z[2 * kk + 1];
+    a[kk][0] = pack_bf16(fmaxf(lo[0], 0.f), fmaxf(lo[1], 0.f));
+    a[kk][1] = pack_bf16(fmaxf(lo[2], 0.f), fmaxf(lo[3], 0.f));
+    a[kk][2] = pack_bf16(fmaxf(hi[0], 0.f), fmaxf(hi[1], 0.f));
+    a[kk][3] = pack_bf16(fmaxf(hi[2], 0.f), fmaxf(hi[3], 0.f));
   }
-#pragma unroll
-  for (int n = 0; n < 8; n++) {
-    const float bl = sm.b2[n * 8 + 2 * t], bh = sm.b2[n * 8 + 2 * t + 1];
-    z2[n][0] = bl;
-    z2[n][1] = bh;
-    z2[n][2] = bl;
-    z2[n][3] = bh;
-#pragma unroll
-    for (int kk = 0; kk < 4; kk++) {
-      uint32_t b0, b1;
-      bfrag(&sm.W2[0][0], W2S, n * 8, kk * 16, g, t, b0, b1);
-      mma_bf16(z2[n], ha[kk][0], ha[kk][1], ha[kk][2], ha[kk][3], b0, b1);
-    }
-  }
-  // layer 3 (64 -> 1) on the CUDA cores: BF16-rounded h2 . w3, reduced over the quad
-  float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-  for (int n = 0; n < 8; n++) {
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const float w = sm.w3[n * 8 + 2 * t + e];
-      s0 += __bfloat162float(__float2bfloat16_rn(fmaxf(z2[n][e], 0.f))) * w;
-      s1 += __bfloat162float(__float2bfloat16_rn(fmaxf(z2[n][2 + e], 0.f))) * w;
-    }
-  }
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-  y0 = s0 + sm.b3;
-  y1 = s1 + sm.b3;
 }
 
 // ----------------------------------------------------------------- inference
@@ -530,168 +518,171 @@ struct GradSmem {
 
 // One CTA = 4 warps = 64-row chunks.  Partial gradients (MLP_P floats) and the loss
 // partial (sum of squared errors) per CTA.  wscale = 2 / (rows in the batch).
+//
+// Bound by instruction issue, not by the tensor cores: operands move between the fragment
+// layouts with ldmatrix and (transposed) stmatrix, four 8x8 matrices at a time, the bias
+// gradients are one more product with ones, and the sums of layer 3 and of the loss stay in
+// each thread until the last chunk.  65,536 rows, cold caches: 25.8 us with 2-byte stores
+// and a scalar loop for the bias sums, 17.2 us in this form (1,024 chunks on 296 CTAs: the
+// fourth turn is half empty).
 __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restrict__ X,
                                                   const float* __restrict__ T, int64_t row0,
                                                   int64_t nrows, const float* __restrict__ P,
                                                   float wscale, float* __restrict__ part,
                                                   float* __restrict__ loss_part) {
-  __shared__ MlpSmem sm;
+  __shared__ __align__(16) MlpSmem sm;
   extern __shared__ __align__(16) unsigned char grad_dyn[];  // GradSmem (> 48 KB static)
   GradSmem& gs = *reinterpret_cast<GradSmem*>(grad_dyn);
-  load_weights(sm, P, gs.W2T);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  for (int i = threadIdx.x; i < 4 * MLP_H; i += blockDim.x) gs.dw3[i / MLP_H][i % MLP_H] = 0.f;
-  if (threadIdx.x < 4) {
-    gs.db3[threadIdx.x] = 0.f;
-    gs.loss[threadIdx.x] = 0.f;
-  }
-  // dW2 rows [16 warp, 16 warp + 16) x 64 cols; dW1 rows [16 warp, +16) x 16 cols
-  float dW2[8][4], dW1[2][4];
+  // inputs and targets of rows g, g + 8 of this warp's 16 rows of a chunk
+  auto load_rows = [&](int64_t ch, uint32_t xa[4], float& ta, float& tb) {
+    const int64_t ra = ch * 64 + warp * 16 + g, rb = ra + 8;
+    const uint32_t* Xa = reinterpret_cast<const uint32_t*>(X + (row0 + ra) * MLP_IN);
+    const uint32_t* Xb = reinterpret_cast<const uint32_t*>(X + (row0 + rb) * MLP_IN);
+    xa[0] = ra < nrows ? __ldg(Xa + t) : 0u;
+    xa[1] = rb < nrows ? __ldg(Xb + t) : 0u;
+    xa[2] = ra < nrows ? __ldg(Xa + t + 4) : 0u;
+    xa[3] = rb < nrows ? __ldg(Xb + t + 4) : 0u;
+    ta = ra < nrows ? __ldg(T + row0 + ra) : 0.f;
+    tb = rb < nrows ? __ldg(T + row0 + rb) : 0.f;
+  };
+  const int64_t nchunks = (nrows + 63) / 64;
+  uint32_t xn[4] = {0u, 0u, 0u, 0u};
+  float tn0 = 0.f, tn1 = 0.f;
+  if (blockIdx.x < nchunks) load_rows(blockIdx.x, xn, tn0, tn1);
+  load_weights(sm, P, gs.W2T);
+  // dW2 rows [16 warp, 16 warp + 16) x 64 cols; dW1 rows [16 warp, +16) x 16 cols; db2 and
+  // db1 of the same rows (every column of the product with ones)
+  float dW2[8][4], dW1[2][4], db2[4], db1[4];
 #pragma unroll
   for (int n = 0; n < 8; n++) dW2[n][0] = dW2[n][1] = dW2[n][2] = dW2[n][3] = 0.f;
 #pragma unroll
   for (int n = 0; n < 2; n++) dW1[n][0] = dW1[n][1] = dW1[n][2] = dW1[n][3] = 0.f;
-  float db1 = 0.f, db2 = 0.f;  // thread i < 64: db2[i]; 64 <= i < 128: db1[i - 64]
-  __syncthreads();
-  const int64_t nchunks = (nrows + 63) / 64;
+#pragma unroll
+  for (int e = 0; e < 4; e++) db2[e] = db1[e] = 0.f;
+  float dw3[8][2], ls = 0.f, bs = 0.f;  // this thread's rows: units 8 n + 2 t + e
+#pragma unroll
+  for (int n = 0; n < 8; n++) dw3[n][0] = dw3[n][1] = 0.f;
   for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    const int64_t r0 = ch * 64 + warp * 16;  // this warp's 16 rows (relative)
-    // inputs of rows r0 + g, r0 + g + 8
-    uint32_t xa[4];
+    uint32_t xa[4] = {xn[0], xn[1], xn[2], xn[3]};
+    const float ta = tn0, tb = tn1;
+    if (ch + gridDim.x < nchunks) load_rows(ch + gridDim.x, xn, tn0, tn1);
+    // ---- forward: z1 -> h1 (fragments) and the signs of z1, z2
+    uint32_t ha[4][4], m1 = 0;
     {
-      const int64_t ra = r0 + g, rb = r0 + g + 8;
-      const uint32_t* Xa = reinterpret_cast<const uint32_t*>(X + (row0 + ra) * MLP_IN);
-      const uint32_t* Xb = reinterpret_cast<const uint32_t*>(X + (row0 + rb) * MLP_IN);
-      xa[0] = ra < nrows ? Xa[t] : 0u;
-      xa[1] = rb < nrows ? Xb[t] : 0u;
-      xa[2] = ra < nrows ? Xa[t + 4] : 0u;
-      xa[3] = rb < nrows ? Xb[t + 4] : 0u;
+      float z1[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t b[4];  // two n-tiles, K = 16
+        ldm4(b, &sm.W1[(n + (lane >> 4)) * 8 + (lane & 7)][((lane >> 3) & 1) * 8]);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const float2 bb = *reinterpret_cast<const float2*>(&sm.b1[(n + q) * 8 + 2 * t]);
+          z1[n + q][0] = z1[n + q][2] = bb.x;
+          z1[n + q][1] = z1[n + q][3] = bb.y;
+          mma_bf16(z1[n + q], xa[0], xa[1], xa[2], xa[3], b[2 * q], b[2 * q + 1]);
+        }
+      }
+      relu_fragments(z1, ha);
+#pragma unroll
+      for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) m1 |= (z1[n][e] > 0.f ? 1u : 0u) << (4 * n + e);
     }
-    float z1[8][4], z2[8][4], y0, y1;
-    mlp_tile_forward(sm, xa, g, t, z1, z2, y0, y1);
-    const int64_t ra = r0 + g, rb = r0 + g + 8;
-    const float e0 = ra < nrows ? y0 - T[row0 + ra] : 0.f;
-    const float e1 = rb < nrows ? y1 - T[row0 + rb] : 0.f;
+    float z2[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+      const float2 bb = *reinterpret_cast<const float2*>(&sm.b2[n * 8 + 2 * t]);
+      z2[n][0] = z2[n][2] = bb.x;
+      z2[n][1] = z2[n][3] = bb.y;
+    }
+    mma_64x64(z2, ha, &sm.W2[0][0], W2S, lane);
+    // layer 3 (64 -> 1) on the CUDA cores: BF16-rounded h2 . w3, reduced over the quad
+    float s0 = 0.f, s1 = 0.f;
+    float h2[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+      const float2 w = *reinterpret_cast<const float2*>(&sm.w3[n * 8 + 2 * t]);
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        h2[n][e] = __bfloat162float(__float2bfloat16_rn(fmaxf(z2[n][e], 0.f)));
+      s0 += h2[n][0] * w.x;
+      s0 += h2[n][1] * w.y;
+      s1 += h2[n][2] * w.x;
+      s1 += h2[n][3] * w.y;
+    }
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+    const int64_t ra = ch * 64 + warp * 16 + g;
+    const float e0 = ra < nrows ? s0 + sm.b3 - ta : 0.f;
+    const float e1 = ra + 8 < nrows ? s1 + sm.b3 - tb : 0.f;
     const float d0 = wscale * e0, d1 = wscale * e1;  // dL/dy
-    {
-      // every lane of a quad holds its rows' errors: sum over the 8 quads of the warp
-      float ls = e0 * e0 + e1 * e1, bs = d0 + d1;
-      ls += __shfl_xor_sync(0xffffffffu, ls, 4);
-      ls += __shfl_xor_sync(0xffffffffu, ls, 8);
-      ls += __shfl_xor_sync(0xffffffffu, ls, 16);
-      bs += __shfl_xor_sync(0xffffffffu, bs, 4);
-      bs += __shfl_xor_sync(0xffffffffu, bs, 8);
-      bs += __shfl_xor_sync(0xffffffffu, bs, 16);
-      if (lane == 0) {
-        gs.loss[warp] += ls;
-        gs.db3[warp] += bs;
-      }
-    }
-    // layer 3 and dZ2 = dy w3 [z2 > 0]
-    float dz2[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int j = n * 8 + 2 * t + e;
-        const float h0 = __bfloat162float(__float2bfloat16_rn(fmaxf(z2[n][e], 0.f)));
-        const float h1v = __bfloat162float(__float2bfloat16_rn(fmaxf(z2[n][2 + e], 0.f)));
-        float pw = d0 * h0 + d1 * h1v;  // dw3[j] partial over rows g, g+8
-        pw += __shfl_xor_sync(0xffffffffu, pw, 4);
-        pw += __shfl_xor_sync(0xffffffffu, pw, 8);
-        pw += __shfl_xor_sync(0xffffffffu, pw, 16);
-        if (g == 0) gs.dw3[warp][j] += pw;
-        dz2[n][e] = z2[n][e] > 0.f ? d0 * sm.w3[j] : 0.f;
-        dz2[n][2 + e] = z2[n][2 + e] > 0.f ? d1 * sm.w3[j] : 0.f;
-      }
-    }
-    // dH1 = dZ2 W2 (A = dZ2 as bf16 fragments, B = W2 via its transpose)
+    ls += e0 * e0 + e1 * e1;
+    bs += d0 + d1;
+    // ---- dw3 and dZ2 = dy w3 [z2 > 0], as fragments
     uint32_t da[4][4];
-#pragma unroll
-    for (int kk = 0; kk < 4; kk++) {
-      da[kk][0] = pack_bf16(dz2[2 * kk][0], dz2[2 * kk][1]);
-      da[kk][1] = pack_bf16(dz2[2 * kk][2], dz2[2 * kk][3]);
-      da[kk][2] = pack_bf16(dz2[2 * kk + 1][0], dz2[2 * kk + 1][1]);
-      da[kk][3] = pack_bf16(dz2[2 * kk + 1][2], dz2[2 * kk + 1][3]);
-    }
-    float dz1[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-      dz1[n][0] = dz1[n][1] = dz1[n][2] = dz1[n][3] = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) {
-        uint32_t b0, b1;
-        bfrag(&gs.W2T[0][0], W2S, n * 8, kk * 16, g, t, b0, b1);
-        mma_bf16(dz1[n], da[kk][0], da[kk][1], da[kk][2], da[kk][3], b0, b1);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; e++) dz1[n][e] = z1[n][e] > 0.f ? dz1[n][e] : 0.f;
-    }
-    // stage transposed tiles (columns = this chunk's 64 rows)
-    const int ca = warp * 16 + g, cb = warp * 16 + g + 8;
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int j = n * 8 + 2 * t + e;
-        gs.dz2T[j][ca] = __float2bfloat16_rn(dz2[n][e]);
-        gs.dz2T[j][cb] = __float2bfloat16_rn(dz2[n][2 + e]);
-        gs.dz1T[j][ca] = __float2bfloat16_rn(dz1[n][e]);
-        gs.dz1T[j][cb] = __float2bfloat16_rn(dz1[n][2 + e]);
-        gs.h1T[j][ca] = __float2bfloat16_rn(fmaxf(z1[n][e], 0.f));
-        gs.h1T[j][cb] = __float2bfloat16_rn(fmaxf(z1[n][2 + e], 0.f));
-      }
-    }
     {
-      const __nv_bfloat162* xa2 = reinterpret_cast<const __nv_bfloat162*>(xa);
-      gs.xT[2 * t][ca] = xa2[0].x;
-      gs.xT[2 * t + 1][ca] = xa2[0].y;
-      gs.xT[2 * t][cb] = xa2[1].x;
-      gs.xT[2 * t + 1][cb] = xa2[1].y;
-      gs.xT[2 * t + 8][ca] = xa2[2].x;
-      gs.xT[2 * t + 9][ca] = xa2[2].y;
-      gs.xT[2 * t + 8][cb] = xa2[3].x;
-      gs.xT[2 * t + 9][cb] = xa2[3].y;
-    }
-    __syncthreads();
-    // dW2[i][j] += sum_r dZ2T[i][r] H1T[j][r];  dW1[i][j] += sum_r dZ1T[i][r] XT[j][r]
-    const int i0 = warp * 16;
-#pragma unroll
-    for (int kk = 0; kk < 4; kk++) {
-      const int k0 = kk * 16;
-      uint32_t a[4], a1[4];
-      a[0] = *reinterpret_cast<const uint32_t*>(&gs.dz2T[i0 + g][k0 + 2 * t]);
-      a[1] = *reinterpret_cast<const uint32_t*>(&gs.dz2T[i0 + g + 8][k0 + 2 * t]);
-      a[2] = *reinterpret_cast<const uint32_t*>(&gs.dz2T[i0 + g][k0 + 2 * t + 8]);
-      a[3] = *reinterpret_cast<const uint32_t*>(&gs.dz2T[i0 + g + 8][k0 + 2 * t + 8]);
-      a1[0] = *reinterpret_cast<const uint32_t*>(&gs.dz1T[i0 + g][k0 + 2 * t]);
-      a1[1] = *reinterpret_cast<const uint32_t*>(&gs.dz1T[i0 + g + 8][k0 + 2 * t]);
-      a1[2] = *reinterpret_cast<const uint32_t*>(&gs.dz1T[i0 + g][k0 + 2 * t + 8]);
-      a1[3] = *reinterpret_cast<const uint32_t*>(&gs.dz1T[i0 + g + 8][k0 + 2 * t + 8]);
 #pragma unroll
       for (int n = 0; n < 8; n++) {
-        uint32_t b0, b1;
-        bfrag(&gs.h1T[0][0], GS, n * 8, k0, g, t, b0, b1);
-        mma_bf16(dW2[n], a[0], a[1], a[2], a[3], b0, b1);
-      }
-#pragma unroll
-      for (int n = 0; n < 2; n++) {
-        uint32_t b0, b1;
-        bfrag(&gs.xT[0][0], GS, n * 8, k0, g, t, b0, b1);
-        mma_bf16(dW1[n], a1[0], a1[1], a1[2], a1[3], b0, b1);
+        const float2 w = *reinterpret_cast<const float2*>(&sm.w3[n * 8 + 2 * t]);
+        dw3[n][0] += d0 * h2[n][0] + d1 * h2[n][2];
+        dw3[n][1] += d0 * h2[n][1] + d1 * h2[n][3];
+        const float a0 = z2[n][0] > 0.f ? d0 * w.x : 0.f, a1 = z2[n][1] > 0.f ? d0 * w.y : 0.f;
+        const float a2 = z2[n][2] > 0.f ? d1 * w.x : 0.f, a3 = z2[n][3] > 0.f ? d1 * w.y : 0.f;
+        da[n >> 1][(n & 1) * 2] = pack_bf16(a0, a1);
+        da[n >> 1][(n & 1) * 2 + 1] = pack_bf16(a2, a3);
       }
     }
-    // bias gradients: thread i < 64 owns db2[i], 64 <= i < 128 owns db1[i - 64]
+    // ---- dH1 = dZ2 W2, dZ1 = dH1 [z1 > 0]
+    uint32_t d1a[4][4];
     {
-      const int i = threadIdx.x & 63;
-      const __nv_bfloat16* rowp = threadIdx.x < 64 ? gs.dz2T[i] : gs.dz1T[i];
-      float sacc = 0.f;
-      for (int c = 0; c < 64; c++) sacc += __bfloat162float(rowp[c]);
-      if (threadIdx.x < 64)
-        db2 += sacc;
-      else
-        db1 += sacc;
+      float dz1[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; n++) dz1[n][0] = dz1[n][1] = dz1[n][2] = dz1[n][3] = 0.f;
+      mma_64x64(dz1, da, &gs.W2T[0][0], W2S, lane);
+#pragma unroll
+      for (int n = 0; n < 8; n++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) dz1[n][e] = (m1 >> (4 * n + e)) & 1u ? dz1[n][e] : 0.f;
+        d1a[n >> 1][(n & 1) * 2] = pack_bf16(dz1[n][0], dz1[n][1]);
+        d1a[n >> 1][(n & 1) * 2 + 1] = pack_bf16(dz1[n][2], dz1[n][3]);
+      }
+    }
+    // ---- stage the transposed tiles (columns = this chunk's 64 rows)
+    const int su = (lane & 7) + ((lane >> 4) & 1) * 8;         // unit of this lane's address
+    const int sc = warp * 16 + ((lane >> 3) & 1) * 8;          // first chunk row of its matrix
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++) {
+      stm4t(&gs.dz2T[kk * 16 + su][sc], da[kk]);
+      stm4t(&gs.dz1T[kk * 16 + su][sc], d1a[kk]);
+      stm4t(&gs.h1T[kk * 16 + su][sc], ha[kk]);
+    }
+    stm4t(&gs.xT[su][sc], xa);
+    __syncthreads();
+    // ---- dW2[i][j] += sum_r dZ2T[i][r] H1T[j][r];  dW1[i][j] += sum_r dZ1T[i][r] XT[j][r]
+    const int i0 = warp * 16;
+    uint32_t a2[4][4], a1[4][4];
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++) {
+      const int ar = i0 + (lane & 7) + ((lane >> 3) & 1) * 8, ac = kk * 16 + (lane >> 4) * 8;
+      ldm4(a2[kk], &gs.dz2T[ar][ac]);
+      ldm4(a1[kk], &gs.dz1T[ar][ac]);
+      constexpr uint32_t ONES = 0x3F803F80u;
+      mma_bf16(db2, a2[kk][0], a2[kk][1], a2[kk][2], a2[kk][3], ONES, ONES);
+      mma_bf16(db1, a1[kk][0], a1[kk][1], a1[kk][2], a1[kk][3], ONES, ONES);
+    }
+    mma_64x64(dW2, a2, &gs.h1T[0][0], GS, lane);
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+      uint32_t b[8];
+      ldm4(b, &gs.xT[n * 8 + (lane & 7)][(lane >> 3) * 8]);
+      ldm4(b + 4, &gs.xT[n * 8 + (lane & 7)][32 + (lane >> 3) * 8]);
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++)
+        mma_bf16(dW1[n], a1[kk][0], a1[kk][1], a1[kk][2], a1[kk][3], b[2 * kk], b[2 * kk + 1]);
     }
     __syncthreads();
   }
@@ -714,10 +705,34 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restric
     out[OFF_W1 + (i0 + g + 8) * MLP_IN + j] = dW1[n][2];
     out[OFF_W1 + (i0 + g + 8) * MLP_IN + j + 1] = dW1[n][3];
   }
-  if (threadIdx.x < 64)
-    out[OFF_B2 + threadIdx.x] = db2;
-  else
-    out[OFF_B1 + threadIdx.x - 64] = db1;
+  if (t == 0) {
+    out[OFF_B2 + i0 + g] = db2[0];
+    out[OFF_B2 + i0 + g + 8] = db2[2];
+    out[OFF_B1 + i0 + g] = db1[0];
+    out[OFF_B1 + i0 + g + 8] = db1[2];
+  }
+  // layer 3 and the loss: over the 8 quads of the warp, then over the warps
+#pragma unroll
+  for (int n = 0; n < 8; n++) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      float pw = dw3[n][e];
+      pw += __shfl_xor_sync(0xffffffffu, pw, 4);
+      pw += __shfl_xor_sync(0xffffffffu, pw, 8);
+      pw += __shfl_xor_sync(0xffffffffu, pw, 16);
+      if (g == 0) gs.dw3[warp][n * 8 + 2 * t + e] = pw;
+    }
+  }
+  ls += __shfl_xor_sync(0xffffffffu, ls, 4);
+  ls += __shfl_xor_sync(0xffffffffu, ls, 8);
+  ls += __shfl_xor_sync(0xffffffffu, ls, 16);
+  bs += __shfl_xor_sync(0xffffffffu, bs, 4);
+  bs += __shfl_xor_sync(0xffffffffu, bs, 8);
+  bs += __shfl_xor_sync(0xffffffffu, bs, 16);
+  if (lane == 0) {
+    gs.loss[warp] = ls;
+    gs.db3[warp] = bs;
+  }
   __syncthreads();
   if (threadIdx.x < MLP_H)
     out[OFF_W3 + threadIdx.x] = ((gs.dw3[0][threadIdx.x] + gs.dw3[1][threadIdx.x]) +
@@ -728,30 +743,49 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const __nv_bfloat16* __restric
   }
 }
 
-// Sum the CTA partials in CTA order, AdamW on the FP32 master parameters.
-__global__ void k_mlp_adamw(const float* __restrict__ part, int nparts,
-                            const float* __restrict__ loss_part, float* __restrict__ P,
-                            float* __restrict__ m, float* __restrict__ v, float lr, float b1,
-                            float b2, float eps, float wd, float bc1, float bc2,
-                            float* __restrict__ grad_out, float* __restrict__ loss_out) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < MLP_P; p += gridDim.x * blockDim.x) {
-    float gsum = 0.f;
-    for (int c = 0; c < nparts; c++) gsum += part[(int64_t)c * MLP_P + p];
-    if (grad_out) grad_out[p] = gsum;
-    if (lr > 0.f) {
-      const float mm = b1 * m[p] + (1.f - b1) * gsum;
-      const float vv = b2 * v[p] + (1.f - b2) * gsum * gsum;
-      m[p] = mm;
-      v[p] = vv;
-      const bool decay = !((p >= OFF_B1 && p < OFF_W2) || (p >= OFF_B2 && p < OFF_W3) ||
-                           p == OFF_B3);
-      P[p] -= lr * ((mm / bc1) / (sqrtf(vv / bc2) + eps) + (decay ? wd * P[p] : 0.f));
-    }
+// Sum the CTA partials, AdamW on the FP32 master parameters.  A block takes 32 parameters
+// (the last block the loss), one per lane; warp w adds the partials w, w + 8, ... and the
+// warps' sums are added in order: a fixed order whatever the schedule, and 8 independent
+// chains of loads per parameter where one thread per parameter walked all of them (bound by
+// the latency of those chains: 296 partials, cold caches, 31 us in that form, 9.5 in this).
+__global__ void __launch_bounds__(256) k_mlp_adamw(
+    const float* __restrict__ part, int nparts, const float* __restrict__ loss_part,
+    float* __restrict__ P, float* __restrict__ m, float* __restrict__ v, float lr, float b1,
+    float b2, float eps, float wd, float bc1, float bc2, float* __restrict__ grad_out,
+    float* __restrict__ loss_out) {
+  __shared__ float s[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool loss = blockIdx.x == gridDim.x - 1;
+  const int p = blockIdx.x * 32 + lane;
+  float acc = 0.f;
+  if (loss) {
+    for (int c = threadIdx.x; c < nparts; c += 256) acc += loss_part[c];
+  } else if (p < MLP_P) {
+#pragma unroll 8
+    for (int c = warp; c < nparts; c += 8) acc += __ldg(part + (int64_t)c * MLP_P + p);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && loss_out) {
-    float l = 0.f;
-    for (int c = 0; c < nparts; c++) l += loss_part[c];
-    *loss_out = l;
+  s[warp][lane] = acc;
+  __syncthreads();
+  if (warp != 0) return;
+  float gsum = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; w++) gsum += s[w][lane];
+  if (loss) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, o);
+    if (lane == 0 && loss_out) *loss_out = gsum;
+    return;
+  }
+  if (p >= MLP_P) return;
+  if (grad_out) grad_out[p] = gsum;
+  if (lr > 0.f) {
+    const float mm = b1 * m[p] + (1.f - b1) * gsum;
+    const float vv = b2 * v[p] + (1.f - b2) * gsum * gsum;
+    m[p] = mm;
+    v[p] = vv;
+    const bool decay = !((p >= OFF_B1 && p < OFF_W2) || (p >= OFF_B2 && p < OFF_W3) ||
+                         p == OFF_B3);
+    P[p] -= lr * ((mm / bc1) / (sqrtf(vv / bc2) + eps) + (decay ? wd * P[p] : 0.f));
   }
 }
 
@@ -861,7 +895,7 @@ extern "C" int tp_mlp_train_step(const void* X, const float* T, int64_t row0, in
   TP_LAUNCH_CHECK();
   const float bc1 = 1.f - powf(beta1, (float)std::max(step, 1));
   const float bc2 = 1.f - powf(beta2, (float)std::max(step, 1));
-  k_mlp_adamw<<<(MLP_P + 255) / 256, 256, 0, st>>>(part, grid, loss_part, params, adam_m, adam_v,
+  k_mlp_adamw<<<(MLP_P + 31) / 32 + 1, 256, 0, st>>>(part, grid, loss_part, params, adam_m, adam_v,
                                                    lr, beta1, beta2, eps, weight_decay, bc1,
                                                    bc2, grad_out, loss_out);
   TP_LAUNCH_CHECK();
