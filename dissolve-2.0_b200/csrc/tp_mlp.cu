@@ -11,7 +11,7 @@
 // B = u^n or the linear extrapolation 2 u^n - u^{n-1} (the network learns the correction
 // to the extrapolation: with zero output the guess is the extrapolation itself).
 //
-// Inference (k_mlp_predict) runs layers 1 and 2 as tcgen05.mma on 128-row tiles with the
+// Inference (k_mlp_predict) runs layers 1 and 2 as tcgen05.mma on 256-row tiles with the
 // accumulators in tensor memory.  Training uses mma.sync.m16n8k16 fragments (row.col,
 // bf16 x bf16 -> f32): a warp owns 16 rows; layer outputs stay in registers and are
 // re-packed from the accumulator layout into the next layer's A layout.  Backward: the
@@ -197,16 +197,20 @@ __device__ __forceinline__ void relu_fragments(const float z[8][4], uint32_t a[4
 }
 
 // ----------------------------------------------------------------- inference
-// 5th-generation tensor cores: 128-row tiles, one row per thread of a 128-thread CTA.
-// Layer 1 (128 x 64, K = 16) and layer 2 (128 x 64, K = 64 as four K = 16 steps) are
-// tcgen05.mma from shared-memory operands into tensor memory (z1 in columns 0..63, z2 in
-// columns 64..127 of a 128-column allocation), issued by one thread and completed through
-// an mbarrier (tcgen05.commit); every thread reads its own row back with tcgen05.ld (warp w
-// owns TMEM lanes 32w..32w+31).  Operands are K-major without swizzle: 8-row x 16-byte
+// 5th-generation tensor cores: 256-row tiles, two rows (128 apart) per thread of a 128-thread
+// CTA.  Layer 1 (128 x 64, K = 16) and layer 2 (128 x 64, K = 64 as four K = 16 steps) of
+// each half are tcgen05.mma from shared-memory operands into tensor memory (64 columns a
+// half; z2 takes z1's columns once every thread has read them), issued by one thread and
+// completed through an mbarrier (tcgen05.commit); every thread reads its own rows back with
+// tcgen05.ld (warp w owns TMEM lanes 32w..32w+31).  Operands are K-major without swizzle: 8-row x 16-byte
 // core matrices, the two 8-element K halves 128 bytes apart, 8-row groups 256 bytes apart.
 // Every mbarrier wait is bounded; a wait that runs out sets the call's status word and
 // g_mlp_tc_timeout, ends the CTA's tiles and still releases its tensor memory.
-constexpr int TC_M = 128, TC_COLS = 128;
+constexpr int TC_M = 128;           // rows of an MMA, threads of a CTA
+constexpr int TC_R = 2;             // rows of a thread: a tile is TC_R MMAs
+constexpr int TC_ROWS = TC_R * TC_M;
+constexpr int TC_COLS = TC_R * MLP_H;  // tensor-memory columns: z1, then z2, of each row
+constexpr int TC_CTAS = 3;          // CTAs of an SM (tensor memory and registers would hold 4)
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 24;  // default polls of one mbarrier phase (~0.1 s)
 
 __device__ int g_mlp_tc_timeout;
@@ -219,11 +223,11 @@ struct TcWait {
 };
 
 struct TcSmem {
-  __nv_bfloat16 A1[TC_M * 16];     // features of the tile, 4 KB
-  __nv_bfloat16 A2[4][TC_M * 16];  // h1 of the tile, one 4 KB block per K step
+  __nv_bfloat16 A1[TC_R][TC_M * 16];     // features of the tile's 128-row parts, 4 KB each
+  __nv_bfloat16 A2[TC_R][4][TC_M * 16];  // their h1, one 4 KB block per K step
   __nv_bfloat16 W1[MLP_H * 16];    // 2 KB
   __nv_bfloat16 W2[4][MLP_H * 16]; // 8 KB
-  float b1[MLP_H], b2[MLP_H], w3[MLP_H];
+  alignas(16) float b1[MLP_H], b2[MLP_H], w3[MLP_H];
   float b3;
   uint64_t bar;
   uint32_t taddr;
@@ -291,47 +295,98 @@ __device__ __forceinline__ void proxy_fence() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// 64 consecutive FP32 columns of this thread's TMEM lane: four loads in flight, one wait
-__device__ __forceinline__ void tc_ld64(uint32_t taddr, float v[64]) {
-  uint32_t r[64];
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-        "%14,%15}, [%16];"
-        : "=r"(r[16 * j + 0]), "=r"(r[16 * j + 1]), "=r"(r[16 * j + 2]), "=r"(r[16 * j + 3]),
-          "=r"(r[16 * j + 4]), "=r"(r[16 * j + 5]), "=r"(r[16 * j + 6]), "=r"(r[16 * j + 7]),
-          "=r"(r[16 * j + 8]), "=r"(r[16 * j + 9]), "=r"(r[16 * j + 10]), "=r"(r[16 * j + 11]),
-          "=r"(r[16 * j + 12]), "=r"(r[16 * j + 13]), "=r"(r[16 * j + 14]), "=r"(r[16 * j + 15])
-        : "r"(taddr + 16u * (uint32_t)j));
+// 16 consecutive FP32 columns of this thread's TMEM lane (tc_ld_wait before their use)
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t r[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+template <int N>
+__device__ __forceinline__ void tc_ld_wait(uint32_t (&r)[N][16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int k = 0; k < 64; k++) v[k] = __uint_as_float(r[k]);
+  for (int k = 0; k < N; k++)
+#pragma unroll
+    for (int i = 0; i < 16; i++) asm volatile("" : "+r"(r[k][i]));
+}
+
+// Two FP32 values in one 64-bit register: packed add and multiply-add (each half rounded on
+// its own, as the scalar operations).
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+// BF16 pair of max(z + b, 0): rounding is monotonic and keeps 0, so the maximum may follow it
+__device__ __forceinline__ uint32_t bias_relu_bf16(uint32_t z0, uint32_t z1, uint64_t b) {
+  const float2 v = f2_unpack(f2_add(f2_pack(__uint_as_float(z0), __uint_as_float(z1)), b));
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
+  asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+  return r;
 }
 
 // x_out[v, s] = B[v, s] + sigma * y(v, s)  (or y_out[r] = y when x_out is NULL).
 // Every thread gathers all features of its row (no divergent per-feature branches).
-__global__ void __launch_bounds__(TC_M) k_mlp_predict(MlpFeat F, int64_t nrows,
+//
+// Bound by the epilogues' instruction issue and shared-memory reads, not by the tensor
+// cores or memory.  So: bias, BF16 rounding and maximum on packed pairs; the biases and w3
+// (16 bytes a read, the same for every lane) read once for two rows; the weights read with
+// every load in flight; one barrier less per tile.  823,875 rows: 50 us with one row per
+// thread and scalar epilogues, 45.7 with packed ones, 36.7 with the weights' loads batched,
+// 32.7 with two rows per thread and 3 CTAs per SM.  (4 CTAs, the most that tensor memory
+// holds: 32.1, but 18.5 instead of 16.6 at 300,000 rows, with more prologues for fewer
+// tiles; one row per thread 20.6 there, and 8.7 instead of 8.3 at 30,000.)
+__global__ void __launch_bounds__(TC_M, TC_CTAS) k_mlp_predict(MlpFeat F, int64_t nrows,
                                                       const float* __restrict__ P, float sigma,
                                                       double* __restrict__ x_out,
                                                       float* __restrict__ y_out, TcWait tw) {
-  __shared__ __align__(128) TcSmem sm;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  TcSmem& sm = *reinterpret_cast<TcSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
   // weights in the operand layout (BF16), biases and w3 (w3 rounded to BF16 as in training)
-  for (int i = tid; i < MLP_H * 16; i += blockDim.x) {
-    const int n = i >> 4, k = i & 15;
-    sm.W1[tc_off(n, k)] = __float2bfloat16_rn(P[OFF_W1 + i]);
-  }
-  for (int i = tid; i < MLP_H * MLP_H; i += blockDim.x) {
-    const int n = i >> 6, k = i & 63;
-    sm.W2[k >> 4][tc_off(n, k & 15)] = __float2bfloat16_rn(P[OFF_W2 + i]);
-  }
+  // (every load of a thread in flight before its first conversion)
+  constexpr int N1 = MLP_H * 16 / TC_M, N2 = MLP_H * MLP_H / TC_M;
+  float w1[N1], w2[N2];
+#pragma unroll
+  for (int k = 0; k < N1; k++) w1[k] = __ldg(P + OFF_W1 + k * TC_M + tid);
+#pragma unroll
+  for (int k = 0; k < N2; k++) w2[k] = __ldg(P + OFF_W2 + k * TC_M + tid);
   for (int i = tid; i < MLP_H; i += blockDim.x) {
     sm.b1[i] = P[OFF_B1 + i];
     sm.b2[i] = P[OFF_B2 + i];
     sm.w3[i] = __bfloat162float(__float2bfloat16_rn(P[OFF_W3 + i]));
   }
   if (tid == 0) sm.b3 = P[OFF_B3];
+#pragma unroll
+  for (int k = 0; k < N1; k++) {
+    const int i = k * TC_M + tid;
+    sm.W1[tc_off(i >> 4, i & 15)] = __float2bfloat16_rn(w1[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < N2; k++) {
+    const int i = k * TC_M + tid, c = i & 63;
+    sm.W2[c >> 4][tc_off(i >> 6, c & 15)] = __float2bfloat16_rn(w2[k]);
+  }
   if (warp == 0) {
     const uint32_t slot = (uint32_t)__cvta_generic_to_shared(&sm.taddr);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot),
@@ -349,116 +404,158 @@ __global__ void __launch_bounds__(TC_M) k_mlp_predict(MlpFeat F, int64_t nrows,
   const uint32_t taddr = sm.taddr;
   const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
   uint32_t phase = 0;
-  const int64_t ntiles = (nrows + TC_M - 1) / TC_M;
-  // (vertex, species) of this thread's row of a tile (vertex 0 past the last row)
-  auto row_of = [&](int64_t tile, int64_t& v, int& s) {
-    const int64_t r = tile * TC_M + tid;
-    // 32-bit division while the row index fits
-    v = r >= nrows ? 0
-                   : (r < (int64_t)UINT32_MAX ? (int64_t)((uint32_t)r / (uint32_t)F.S) : r / F.S);
-    s = r >= nrows ? 0 : (int)(r - v * F.S);
+  constexpr int R = TC_R;
+  const int64_t ntiles = (nrows + TC_ROWS - 1) / TC_ROWS;
+  // (vertex, species) of this thread's first row, advanced by a grid of rows from tile to
+  // tile; row k of the thread is 128 k rows on
+  const int64_t step = (int64_t)gridDim.x * TC_ROWS, dv = step / F.S;
+  const int ds = (int)(step - dv * F.S), dvk = TC_M / F.S, dsk = TC_M - dvk * F.S;
+  int64_t r = (int64_t)blockIdx.x * TC_ROWS + tid, v = r / F.S;
+  int s = (int)(r - v * F.S);
+  auto advance = [&](int64_t& vv, int& ss, int64_t a, int b) {
+    vv += a;
+    ss += b;
+    if (ss >= F.S) {
+      ss -= F.S;
+      vv++;
+    }
+  };
+  RowFields cur[R];
+  auto load_rows = [&]() {
+    int64_t vk = v;
+    int sk = s;
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      cur[k] = RowFields{};
+      if (r + k * TC_M < nrows) cur[k] = row_fields(F, vk, sk);
+      advance(vk, sk, dvk, dsk);
+    }
   };
   // the fields of the CTA's first tile; every tile's MMAs overlap the next tile's loads
-  RowFields cur{};
-  if (blockIdx.x < ntiles) {
-    int64_t v0;
-    int s0;
-    row_of(blockIdx.x, v0, s0);
-    cur = row_fields(F, v0, s0);
-  }
+  load_rows();
+  bool ok = true;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t r = tile * TC_M + tid;
-    const bool in = r < nrows;
-    int64_t v;
-    int s;
-    row_of(tile, v, s);
+    bool in[R];
+    double base[R];
+    int64_t out[R];
     {
-      float f[NFEAT];
-      fields_features(F, cur, s, f);
-      uint32_t w[8];
+      int64_t vk = v;
+      int sk = s;
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const float lo = (in && 2 * k < NFEAT) ? f[2 * k] : 0.f;
-        const float hi = (in && 2 * k + 1 < NFEAT) ? f[2 * k + 1] : 0.f;
-        w[k] = pack_bf16(lo, hi);
+      for (int q = 0; q < R; q++) {
+        in[q] = r + q * TC_M < nrows;
+        float f[NFEAT];
+        fields_features(F, cur[q], sk, f);
+        uint32_t w[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const float lo = (in[q] && 2 * k < NFEAT) ? f[2 * k] : 0.f;
+          const float hi = (in[q] && 2 * k + 1 < NFEAT) ? f[2 * k + 1] : 0.f;
+          w[k] = pack_bf16(lo, hi);
+        }
+        __nv_bfloat16* A = sm.A1[q];
+        *reinterpret_cast<uint4*>(A + tc_off(tid, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(A + tc_off(tid, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+        base[q] = F.base == 1 ? 2.0 * cur[q].u - cur[q].up : (F.base == 0 ? cur[q].u : 0.0);
+        out[q] = x_out ? vk * F.ld + sk : r + q * TC_M;
+        advance(vk, sk, dvk, dsk);
       }
-      *reinterpret_cast<uint4*>(&sm.A1[tc_off(tid, 0)]) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(&sm.A1[tc_off(tid, 8)]) = make_uint4(w[4], w[5], w[6], w[7]);
     }
     proxy_fence();
     tc_fence_before();
-    __syncthreads();
+    // also: every thread's reads of the last tile's z2 are done
+    if (__syncthreads_or(!ok)) break;
     tc_fence_after();
     if (tid == 0 && !tw.skip_issue) {
-      tc_mma(taddr, tc_desc(sm.A1), tc_desc(sm.W1), 0);
+#pragma unroll
+      for (int q = 0; q < R; q++)
+        tc_mma(taddr + q * MLP_H, tc_desc(sm.A1[q]), tc_desc(sm.W1), 0);
       tc_commit(&sm.bar);
     }
-    RowFields nxt{};
-    if (tile + gridDim.x < ntiles) {
-      int64_t vn;
-      int sn;
-      row_of(tile + gridDim.x, vn, sn);
-      nxt = row_fields(F, vn, sn);
-    }
-    bool ok = tc_wait(&sm.bar, phase, tw.polls);
+    r += step;
+    advance(v, s, dv, ds);
+    load_rows();
+    ok = tc_wait(&sm.bar, phase, tw.polls);
     phase ^= 1u;
     tc_fence_after();
-    // h1 = relu(z1 + b1), BF16, into the layer-2 operand
-    float z1[64];
-    tc_ld64(taddr + lane_base, z1);
+    // h1 = relu(z1 + b1), BF16, into the layer-2 operand: 16 columns at a time
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const float* z = z1 + 16 * j;
-      uint32_t w[8];
+      uint32_t z[R][16];
 #pragma unroll
-      for (int k = 0; k < 8; k++)
-        w[k] = pack_bf16(fmaxf(z[2 * k] + sm.b1[16 * j + 2 * k], 0.f),
-                         fmaxf(z[2 * k + 1] + sm.b1[16 * j + 2 * k + 1], 0.f));
-      *reinterpret_cast<uint4*>(&sm.A2[j][tc_off(tid, 0)]) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(&sm.A2[j][tc_off(tid, 8)]) = make_uint4(w[4], w[5], w[6], w[7]);
+      for (int q = 0; q < R; q++) tc_ld16(taddr + lane_base + q * MLP_H + 16 * j, z[q]);
+      tc_ld_wait(z);
+      uint32_t w[R][8];
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(&sm.b1[16 * j + 2 * k]);
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          w[q][k] = bias_relu_bf16(z[q][2 * k], z[q][2 * k + 1], bb.x);
+          w[q][k + 1] = bias_relu_bf16(z[q][2 * k + 2], z[q][2 * k + 3], bb.y);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        __nv_bfloat16* A = sm.A2[q][j];
+        *reinterpret_cast<uint4*>(A + tc_off(tid, 0)) =
+            make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+        *reinterpret_cast<uint4*>(A + tc_off(tid, 8)) =
+            make_uint4(w[q][4], w[q][5], w[q][6], w[q][7]);
+      }
     }
     proxy_fence();
     tc_fence_before();
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) tc_timed_out(tw);
-      break;
-    }
+    if (__syncthreads_or(!ok)) break;
     tc_fence_after();
-    if (tid == 0 && !tw.skip_issue) {
+    if (tid == 0 && !tw.skip_issue) {  // every thread has read z1: z2 takes its columns
 #pragma unroll
-      for (int j = 0; j < 4; j++) tc_mma(taddr + MLP_H, tc_desc(sm.A2[j]), tc_desc(sm.W2[j]), j > 0);
+      for (int q = 0; q < R; q++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          tc_mma(taddr + q * MLP_H, tc_desc(sm.A2[q][j]), tc_desc(sm.W2[j]), j > 0);
       tc_commit(&sm.bar);
     }
     ok = tc_wait(&sm.bar, phase, tw.polls);
     phase ^= 1u;
     tc_fence_after();
     // layer 3 on the CUDA cores: BF16-rounded h2 . w3 + b3
-    float y = 0.f;
-    {
-      float z2[64];
-      tc_ld64(taddr + lane_base + MLP_H, z2);
+    uint64_t acc[R][2];
 #pragma unroll
-      for (int k = 0; k < 64; k++)
-        y += __bfloat162float(__float2bfloat16_rn(fmaxf(z2[k] + sm.b2[k], 0.f))) * sm.w3[k];
-    }
-    y += sm.b3;
-    if (in && ok) {
-      if (x_out) {
-        const int64_t i = v * F.ld + s;
-        const double b = F.base == 1 ? 2.0 * cur.u - cur.up : (F.base == 0 ? cur.u : 0.0);
-        x_out[i] = b + (double)sigma * (double)y;
-      } else {
-        y_out[r] = y;
+    for (int q = 0; q < R; q++) acc[q][0] = acc[q][1] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      uint32_t z[R][16];
+#pragma unroll
+      for (int q = 0; q < R; q++) tc_ld16(taddr + lane_base + q * MLP_H + 16 * j, z[q]);
+      tc_ld_wait(z);
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) {
+        const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(&sm.b2[16 * j + k]);
+        const ulonglong2 ww = *reinterpret_cast<const ulonglong2*>(&sm.w3[16 * j + k]);
+        auto h2 = [](uint32_t p) {
+          return f2_pack(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+        };
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          acc[q][0] = f2_fma(h2(bias_relu_bf16(z[q][k], z[q][k + 1], bb.x)), ww.x, acc[q][0]);
+          acc[q][1] = f2_fma(h2(bias_relu_bf16(z[q][k + 2], z[q][k + 3], bb.y)), ww.y, acc[q][1]);
+        }
       }
     }
-    // the tile's tensor-memory reads and operand reads are done before the next tile
-    tc_fence_before();
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) tc_timed_out(tw);
-      break;
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      const float2 p = f2_unpack(f2_add(acc[q][0], acc[q][1]));
+      const float y = p.x + p.y + sm.b3;
+      if (in[q] && ok) {
+        if (x_out)
+          x_out[out[q]] = base[q] + (double)sigma * (double)y;
+        else
+          y_out[out[q]] = y;
+      }
     }
-    cur = nxt;
   }
+  if (!ok) tc_timed_out(tw);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -827,13 +924,15 @@ extern "C" int tp_mlp_predict(const tp_mlp_inputs* in, const float* params, floa
   TP_REQUIRE(in->base >= 0 && in->base <= 2, "base must be 0 (u^n), 1 (2 u^n - u^{n-1}) or 2 (none)");
   const int64_t nrows = in->n_verts * in->S;
   if (nrows == 0) return TP_OK;
-  const int64_t ntiles = (nrows + TC_M - 1) / TC_M;
-  // persistent CTAs, 4 per SM (4 x 128 tensor-memory columns = the SM's 512)
-  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * 4);
   cudaStream_t st = as_stream(stream);
   TcWait tw{g_tc_polls.load(), g_tc_skip.load(), in->tc_status};
   if (tw.status) TP_CUDA_TRY(cudaMemsetAsync(tw.status, 0, sizeof(int32_t), st));
-  k_mlp_predict<<<grid, TC_M, 0, st>>>(make_feat(in), nrows, params, sigma, x_out, y_out, tw);
+  const int64_t ntiles = (nrows + TC_ROWS - 1) / TC_ROWS;
+  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * TC_CTAS);
+  TP_CUDA_TRY(cudaFuncSetAttribute(k_mlp_predict, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(TcSmem)));
+  k_mlp_predict<<<grid, TC_M, sizeof(TcSmem), st>>>(make_feat(in), nrows, params, sigma, x_out,
+                                                    y_out, tw);
   TP_LAUNCH_CHECK();
   return TP_OK;
 }
