@@ -43,6 +43,11 @@
 // latency per exchange, where a grid barrier costs an arrival, a poll and then the load.
 // The buffers are cleared before a solve, so an old number is never taken for a new one; a
 // unit is rewritten only after its readers have sent the sums that the writer waits for.
+// Past two rows a thread, three or four FP32 columns are laid out for it in another way
+// (cc_planes): planes in shared memory, the vectors in tensor memory.  The product is bound
+// by shared-memory bandwidth there: 274,625 rows of three columns, us per iteration: 10.0
+// with rows padded to 16 bytes and vectors spilled past the registers, 8.6 with planes, 6.5
+// once one column is left (columns of larger diffusion take half as many passes more).
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -271,6 +276,23 @@ __device__ __forceinline__ void cc_tm_ld16(uint32_t t, uint32_t r[16]) {
       : "r"(t)
       : "memory");
 }
+__device__ __forceinline__ void cc_tm_st4(uint32_t t, const uint32_t v[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(t), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+__device__ __forceinline__ void cc_tm_ld4(uint32_t t, uint32_t r[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(t)
+               : "memory");
+}
+__device__ __forceinline__ void cc_tm_ld1(uint32_t t, uint32_t& r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(t) : "memory");
+}
+__device__ __forceinline__ void cc_tm_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cc_tm_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -380,6 +402,15 @@ __device__ __forceinline__ void axpy_row(VT v, const VT u[LD], VT y[LD]) {
   }
 }
 
+// Whether a system over all SMs keeps its rows in planes and its vectors in tensor memory
+// (k_ccg): three or four FP32 columns and more than two rows a thread, whose vectors do not
+// fit the registers (three columns, us per iteration at 274,625 rows: 10.1 with 16-byte
+// rows and spilled vectors, 8.7 with planes; at 117,649, two rows a thread: 6.1 and 6.4).
+template <typename VT>
+constexpr bool cc_planes(int NC, int RPT, bool grid) {
+  return grid && sizeof(VT) == 4 && NC >= 3 && RPT > 2;
+}
+
 // RPT: slices per warp (rows per thread).  Dynamic shared memory: two buffers of partial
 // sums (16 CTAs x 16), the window (win_cap rows), w, then this part's slice offsets, push
 // list, diagonal, columns and values, each where it still fits.
@@ -394,10 +425,44 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   __shared__ uint32_t s_taddr;
   __shared__ volatile int s_gave_up;
   // what warp 0 decided for the next pass (Ctl bits, refreshed columns) and its coefficients
-  __shared__ int s_ctl, s_mask;
+  __shared__ int s_ctl, s_mask, s_run;
   __shared__ VT s_al[4], s_be[4];
   enum : int { CTL_REFRESH = 1, CTL_FIN = 2, CTL_EXIT = 4 };
-  constexpr int RB = LD * (int)sizeof(VT);
+  // PL: the window, w and the diagonal in planes, 32 values of a column side by side (row i,
+  // column s at (i / 32) 32 NC + 32 s + i % 32): a column of 32 neighbouring rows is one
+  // 128-byte access, and no room or bandwidth goes to a padding column.  The vectors of a
+  // row are then kept in tensor memory, 16 words per slice next to the values: word 4 s
+  // + 0..3 r, p, q, xi of column s, word 12 + s D^-1 (four columns: D^-1 in registers).
+  constexpr bool PL = cc_planes<VT>(NC, RPT, GRID);
+  // ONE: once a single column still runs, a pass computes and exchanges that column only
+  // (three columns at 274,625 rows: 6.5 us a pass instead of 8.7; with 16-byte rows, where
+  // such a pass reads as much shared memory as a full one, it gains less than the second
+  // code path costs the full passes: 4 % at 117,649 rows)
+  constexpr bool ONE = PL;
+  static_assert(!PL || RPT <= 4, "tensor memory: 16 words of values and 16 of vectors a slice");
+  constexpr int RB = PL ? NC * (int)sizeof(VT) : LD * (int)sizeof(VT);
+  auto padded = [](int n) { return PL ? (n + 31) & ~31 : n; };
+  auto w_ld = [](const VT* w, int i, VT v[LD]) {
+    if constexpr (PL) {
+      const VT* q = w + (i >> 5) * 32 * NC + (i & 31);
+#pragma unroll
+      for (int s = 0; s < LD; s++) v[s] = s < NC ? q[32 * (s < NC ? s : 0)] : VT(0);
+    } else {
+      lds_row<VT, LD>(w, i, v);
+    }
+  };
+  auto w_st = [](VT* w, int i, const VT v[LD]) {
+    if constexpr (PL) {
+      VT* q = w + (i >> 5) * 32 * NC + (i & 31);
+#pragma unroll
+      for (int s = 0; s < NC; s++) q[32 * s] = v[s];
+    } else {
+      sts_row<VT, LD>(w, i, v);
+    }
+  };
+  auto w_at = [](int i, int s) {  // where column s of row i is
+    return PL ? (i >> 5) * 32 * NC + 32 * s + (i & 31) : i * LD + s;
+  };
   constexpr int VW = (int)sizeof(VT) / 4;             // 32-bit words of a value
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = GRID ? blockIdx.x : cl_rank(), C = GRID ? gridDim.x : cl_size();
@@ -476,11 +541,11 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       top += bytes;
       return at;
     };
-    VT* const s_w = reinterpret_cast<VT*>(s_dyn + carve(nrows * RB));
+    VT* const s_w = reinterpret_cast<VT*>(s_dyn + carve(padded(nrows) * RB));
     int32_t* const s_sl = reinterpret_cast<int32_t*>(s_dyn + carve(4 * (part.nslices + 1)));
     // the rows to push (GRID: the halo rows to poll)
     uint32_t* const s_push = reinterpret_cast<uint32_t*>(s_dyn + carve(4 * part.npush));
-    const int o_diag = a.diag ? carve(nrows * RB) : -1;
+    const int o_diag = a.diag ? carve(padded(nrows) * RB) : -1;
     const int o_col = carve(2 * part.entries);
     const uint16_t* const g_col = a.loc_col + part.entry_off;
     for (int i = tid; i <= part.nslices; i += CC_T) s_sl[i] = a.slices[part.slice_off + i];
@@ -489,9 +554,18 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     if (o_col >= 0)
       for (int i = tid; i < part.entries / 8; i += CC_T)
         reinterpret_cast<uint4*>(s_dyn + o_col)[i] = reinterpret_cast<const uint4*>(g_col)[i];
-    if (o_diag >= 0)
-      for (int i = tid; i < nrows * LD; i += CC_T)
-        reinterpret_cast<VT*>(s_dyn + o_diag)[i] = a.diag[row0 * LD + i];
+    if (o_diag >= 0) {
+      VT* const d = reinterpret_cast<VT*>(s_dyn + o_diag);
+      if constexpr (PL) {
+        for (int i = tid; i < nrows; i += CC_T) {
+          VT t[LD];
+          ldv<VT, LD>(a.diag, row0 + i, t);
+          w_st(d, i, t);
+        }
+      } else {
+        for (int i = tid; i < nrows * LD; i += CC_T) d[i] = a.diag[row0 * LD + i];
+      }
+    }
     __syncthreads();
     const int v0 = s_sl[part.val_slice];  // first entry whose value is not in tensor memory
     const int o_val = o_col >= 0 ? carve((int)sizeof(VT) * (part.entries - v0)) : -1;
@@ -536,10 +610,57 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         }
       }
     }
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    cc_tm_wait_st();
 
-    // rows of this thread: slice warp + 16 i, lane
-    VT r[RPT][NC], p[RPT][NC], q[RPT][NC], xi[RPT][NC], dv[RPT][NC];
+    // rows of this thread: slice warp + 16 i, lane.  In registers, or (PL) in tensor memory:
+    // loads (all lanes, then vec_wait) and stores are copies, a register form's cost nothing.
+    struct Vec {
+      VT r[NC], p[NC], q[NC], xi[NC], dv[NC];
+    };
+    constexpr bool DV = PL && NC <= 3;  // D^-1 in tensor memory
+    Vec vec[PL ? 1 : RPT] = {};
+    VT dvr[PL && !DV ? RPT : 1][NC];
+    const uint32_t tv0 = tm + 64u;
+    auto vec_ld = [&](int i, uint32_t t[16]) {
+      if constexpr (PL) cc_tm_ld16(tv0 + 16u * (uint32_t)i, t);
+    };
+    auto vec_get = [&](int i, const uint32_t t[16], Vec& v) {
+      if constexpr (PL) {
+#pragma unroll
+        for (int s = 0; s < NC; s++) {
+          v.r[s] = __uint_as_float(t[4 * s]);
+          v.p[s] = __uint_as_float(t[4 * s + 1]);
+          v.q[s] = __uint_as_float(t[4 * s + 2]);
+          v.xi[s] = __uint_as_float(t[4 * s + 3]);
+          if constexpr (DV)
+            v.dv[s] = __uint_as_float(t[(12 + s) & 15]);
+          else
+            v.dv[s] = dvr[i][s];
+        }
+      } else {
+        v = vec[i];
+      }
+    };
+    auto vec_put = [&](int i, const Vec& v) {
+      if constexpr (PL) {
+        uint32_t t[16];
+        t[15] = 0u;
+#pragma unroll
+        for (int s = 0; s < NC; s++) {
+          t[4 * s] = __float_as_uint(v.r[s]);
+          t[4 * s + 1] = __float_as_uint(v.p[s]);
+          t[4 * s + 2] = __float_as_uint(v.q[s]);
+          t[4 * s + 3] = __float_as_uint(v.xi[s]);
+          if constexpr (DV) t[(12 + s) & 15] = __float_as_uint(v.dv[s]);
+        }
+        cc_tm_st16(tv0 + 16u * (uint32_t)i, t);
+      } else {
+        vec[i] = v;
+      }
+    };
+    auto vec_wait = [&]() {
+      if constexpr (PL) cc_tm_wait_ld();
+    };
     // ---- Jacobi diagonal (FP64 values) through s_w; Dirichlet values into x
     for (int sl = warp; sl < part.nslices; sl += CC_W) {
       const int lr = sl * 32 + lane;
@@ -558,11 +679,11 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           d[s] = (s < S && !bcr && t != 0.0) ? VT(1.0 / t) : VT(0);
           if (bcr) a.x[row * LD + s] = a.b[row * LD + s];
         }
-        sts_row<VT, LD>(s_w, lr, d);
+        w_st(s_w, lr, d);
         VT z[LD];
 #pragma unroll
         for (int s = 0; s < LD; s++) z[s] = VT(0);
-        sts_row<VT, LD>(s_win, lr, z);
+        w_st(s_win, lr, z);
       }
     }
 #pragma unroll
@@ -571,13 +692,17 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       VT t[LD];
 #pragma unroll
       for (int s = 0; s < LD; s++) t[s] = VT(0);
-      if (lr < nrows) lds_row<VT, LD>(s_w, lr, t);
+      if (lr < nrows) w_ld(s_w, lr, t);
+      Vec v;
 #pragma unroll
       for (int s = 0; s < NC; s++) {
-        r[i][s] = p[i][s] = q[i][s] = xi[i][s] = VT(0);
-        dv[i][s] = t[s];
+        v.r[s] = v.p[s] = v.q[s] = v.xi[s] = VT(0);
+        v.dv[s] = t[s];
+        if constexpr (PL && !DV) dvr[i][s] = t[s];
       }
+      vec_put(i, v);
     }
+    if constexpr (PL) cc_tm_wait_st();
 
     // lane state: lane s < S of warp 0 holds column s (the same bits in every CTA)
     const int col = lane & 3;
@@ -589,6 +714,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     int st_act = 0, st_frozen = 0, st_status = TP_OK, st_iters = 0;
     unsigned tr_mask = (1u << S) - 1;  // columns refreshed by the next FP64 sweep
     bool refresh = true, first = true, fin = false;
+    int one = -1;  // ONE: the only column that still runs (the others stand still), or -1
     int it = 0, n_rel = 0;
 
     for (;;) {
@@ -600,19 +726,26 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
 #pragma unroll
         for (int i = 0; i < RPT; i++) {
           const int lr = (warp + i * CC_W) * 32 + lane;
+          uint32_t tw[16];
+          Vec v;
+          vec_ld(i, tw);
+          vec_wait();
+          vec_get(i, tw, v);
           if (lr < nrows) {
             const int64_t row = row0 + lr;
             VT t[LD];
 #pragma unroll
-            for (int s = 0; s < LD; s++) t[s] = s < NC ? r[i][s] : VT(0);
-            sts_row<VT, LD>(s_w, lr, t);
+            for (int s = 0; s < LD; s++) t[s] = s < NC ? v.r[s < NC ? s : 0] : VT(0);
+            w_st(s_w, lr, t);
 #pragma unroll
             for (int s = 0; s < NC; s++) {
-              if (((tr_mask >> s) & 1) && !first) a.x[row * LD + s] += (double)xi[i][s];
-              if ((tr_mask >> s) & 1) xi[i][s] = VT(0);
+              if (((tr_mask >> s) & 1) && !first) a.x[row * LD + s] += (double)v.xi[s];
+              if ((tr_mask >> s) & 1) v.xi[s] = VT(0);
             }
           }
+          vec_put(i, v);
         }
+        if constexpr (PL) cc_tm_wait_st();
         x_sync();
         // a slice at a time: 8 lanes walk a row (coalesced index and value loads, 4 rows per
         // step, the steps' loads in flight together), the sums go to the rows' own lanes
@@ -670,7 +803,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           }
           if (in) {
             VT rv[LD];
-            lds_row<VT, LD>(s_w, lr, rv);
+            w_ld(s_w, lr, rv);
 #pragma unroll
             for (int s = 0; s < NC; s++) {
               const double dd = (a.A64.diag && !bcr) ? a.A64.diag[row * LD + s] : 0.0;
@@ -681,7 +814,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
               if (fin || ((tr_mask >> s) & 1)) rr[s] += r64 * r64;
               if (!fin && ((tr_mask >> s) & 1)) rv[s] = (VT)r64;
             }
-            sts_row<VT, LD>(s_w, lr, rv);
+            w_st(s_w, lr, rv);
           }
         }
         if (first) {
@@ -697,19 +830,69 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
 #pragma unroll
         for (int i = 0; i < RPT; i++) {
           const int lr = (warp + i * CC_W) * 32 + lane;
+          uint32_t tw[16];
+          Vec v;
+          vec_ld(i, tw);
+          vec_wait();
+          vec_get(i, tw, v);
           if (lr < nrows) {
             VT uv[LD], rv[LD];
-            lds_row<VT, LD>(s_win, lr, uv);
-            lds_row<VT, LD>(s_w, lr, rv);
+            w_ld(s_win, lr, uv);
+            w_ld(s_w, lr, rv);
 #pragma unroll
             for (int s = 0; s < NC; s++) {
-              r[i][s] = rv[s];
-              if (!fin && ((tr_mask >> s) & 1)) uv[s] = dv[i][s] * r[i][s];
-              acc[s] += (double)r[i][s] * (double)uv[s];
+              v.r[s] = rv[s];
+              if (!fin && ((tr_mask >> s) & 1)) uv[s] = v.dv[s] * v.r[s];
+              acc[s] += (double)v.r[s] * (double)uv[s];
             }
-            sts_row<VT, LD>(s_win, lr, uv);
+            w_st(s_win, lr, uv);
             publish(row0 + lr, uv);
           }
+          vec_put(i, v);
+        }
+        if constexpr (PL) cc_tm_wait_st();
+      } else if (ONE && one >= 0) {
+        // ---- the same for the one column that still runs
+        if constexpr (ONE) {
+          uint32_t tw[RPT][4], td[RPT];
+#pragma unroll
+          for (int i = 0; i < RPT; i++) {
+            cc_tm_ld4(tv0 + 16u * (uint32_t)i + 4u * (uint32_t)one, tw[i]);
+            if constexpr (DV) cc_tm_ld1(tv0 + 16u * (uint32_t)i + 12u + (uint32_t)one, td[i]);
+          }
+          const float al = s_al[one], be = s_be[one];
+          cc_tm_wait_ld();
+          // D^-1 of a register form
+          auto sel = [&](const VT* v) {
+            VT t = v[0];
+#pragma unroll
+            for (int s = 1; s < NC; s++) t = one == s ? v[s] : t;
+            return t;
+          };
+#pragma unroll
+          for (int i = 0; i < RPT; i++) {
+            const int sl = warp + i * CC_W, lr = sl * 32 + lane;
+            const int at = w_at(lr, one);
+            float r = __uint_as_float(tw[i][0]), p = __uint_as_float(tw[i][1]),
+                  q = __uint_as_float(tw[i][2]), xi = __uint_as_float(tw[i][3]);
+            const float dv = DV ? __uint_as_float(td[i]) : sel(dvr[DV ? 0 : i]);
+            if (lr < nrows) {
+              p = s_win[at] + be * p;
+              q = s_w[at] + be * q;
+              xi += al * p;
+              r -= al * q;
+              const float u = dv * r;
+              acc[0] += (double)r * (double)u;
+              acc[1] += (double)r * (double)r;
+              s_win[at] = u;
+              st_unit(a.ubuf + (row0 + lr) * UW, (unsigned long long)__float_as_uint(u),
+                      (unsigned long long)epoch << 32);
+            }
+            const uint32_t t[4] = {__float_as_uint(r), __float_as_uint(p), __float_as_uint(q),
+                                   __float_as_uint(xi)};
+            cc_tm_st4(tv0 + 16u * (uint32_t)i + 4u * (uint32_t)one, t);
+          }
+          cc_tm_wait_st();
         }
       } else {
         // ---- vector update with this iteration's alpha and beta
@@ -719,27 +902,37 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           al[s] = s_al[s];
           be[s] = s_be[s];
         }
+        uint32_t tw[PL ? RPT : 1][16];
+        if constexpr (PL) {
+#pragma unroll
+          for (int i = 0; i < RPT; i++) vec_ld(i, tw[i]);
+          vec_wait();
+        }
 #pragma unroll
         for (int i = 0; i < RPT; i++) {
           const int lr = (warp + i * CC_W) * 32 + lane;
+          Vec v;
+          vec_get(i, tw[PL ? i : 0], v);
           if (lr < nrows) {
             VT uv[LD], wv[LD];
-            lds_row<VT, LD>(s_win, lr, uv);
-            lds_row<VT, LD>(s_w, lr, wv);
+            w_ld(s_win, lr, uv);
+            w_ld(s_w, lr, wv);
 #pragma unroll
             for (int s = 0; s < NC; s++) {
-              p[i][s] = uv[s] + be[s] * p[i][s];
-              q[i][s] = wv[s] + be[s] * q[i][s];
-              xi[i][s] += al[s] * p[i][s];
-              r[i][s] -= al[s] * q[i][s];
-              uv[s] = dv[i][s] * r[i][s];
-              acc[s] += (double)r[i][s] * (double)uv[s];
-              acc[NC + s] += (double)r[i][s] * (double)r[i][s];
+              v.p[s] = uv[s] + be[s] * v.p[s];
+              v.q[s] = wv[s] + be[s] * v.q[s];
+              v.xi[s] += al[s] * v.p[s];
+              v.r[s] -= al[s] * v.q[s];
+              uv[s] = v.dv[s] * v.r[s];
+              acc[s] += (double)v.r[s] * (double)uv[s];
+              acc[NC + s] += (double)v.r[s] * (double)v.r[s];
             }
-            sts_row<VT, LD>(s_win, lr, uv);
+            w_st(s_win, lr, uv);
             publish(row0 + lr, uv);
           }
+          vec_put(i, v);
         }
+        if constexpr (PL) cc_tm_wait_st();
       }
       // ---- the rows other CTAs hold as halo, then (while they travel) this warp's r.u, r.r
       __syncthreads();
@@ -754,7 +947,11 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
                           cl_map(&s_mb[2], dst));
         }
       }
-      {
+      if (ONE && one >= 0) {
+        const double v = WarpReduce<2>::run(acc, lane);
+        const int id = WarpReduce<2>::value_of(lane);
+        if (id >= 0) s_red[warp][4 * id + one] = v;
+      } else {
         const double v = WarpReduce<2 * NC>::run(acc, lane);
         const int id = WarpReduce<2 * NC>::value_of(lane);
         if (id >= 0) s_red[warp][(id / NC) * 4 + id % NC] = v;
@@ -763,6 +960,26 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       if constexpr (GRID) {
         const uint32_t want = epoch + a.wait_missing;
         constexpr int U = UW == 1 ? 8 : (UW == 2 ? 4 : 2);
+        if (ONE && one >= 0) {
+          for (int i0 = tid; i0 < part.nhalo; i0 += 8 * CC_T) {
+            ulonglong2 v[8];
+            const ulonglong2* src[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              src[k] = a.ubuf + (int64_t)s_push[min(i0 + k * CC_T, part.nhalo - 1)] * UW;
+              v[k] = ld_unit(src[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              if (i0 + k * CC_T < part.nhalo) {
+                if (!poll_unit<TAG>(src[k], v[k], want, a.wait_limit_ns, &s_gave_up)) s_gave_up = 1;
+                const int i = nrows + i0 + k * CC_T;
+                const uint32_t w = (uint32_t)v[k].x;
+                memcpy(s_win + w_at(i, one), &w, 4);
+              }
+            }
+          }
+        } else
         for (int i0 = tid; i0 < part.nhalo; i0 += U * CC_T) {
           ulonglong2 v[U][UW];
           const ulonglong2* src[U];
@@ -793,7 +1010,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
                     if (3 * j + s < LD) uv[3 * j + s] = __uint_as_float(w[s]);
                 }
               }
-              sts_row<VT, LD>(s_win, nrows + i0 + k * CC_T, uv);
+              w_st(s_win, nrows + i0 + k * CC_T, uv);
             }
           }
         }
@@ -807,50 +1024,82 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       double wu[NC];
 #pragma unroll
       for (int s = 0; s < NC; s++) wu[s] = 0.0;
-      // columns are byte offsets into the window (GRID: its entries)
-      constexpr uint32_t CU = GRID ? RB : 1;
-      const unsigned char* const s_winb = reinterpret_cast<const unsigned char*>(s_win);
-      auto gather4 = [&](uint2 c, const VT* v, VT ak[LD], VT ak2[LD]) {
-        VT u0[LD], u1[LD], u2[LD], u3[LD];
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x & 0xffffu) * CU), 0, u0);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.x >> 16) * CU), 0, u1);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y & 0xffffu) * CU), 0, u2);
-        lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + (c.y >> 16) * CU), 0, u3);
-        axpy_row<VT, LD>(v[0], u0, ak);
-        axpy_row<VT, LD>(v[1], u1, ak2);
-        axpy_row<VT, LD>(v[2], u2, ak);
-        axpy_row<VT, LD>(v[3], u3, ak2);
+      // columns are byte offsets into the window (GRID: its entries; PL: its words).
+      // N: columns computed, NC or (one column left) 1
+      constexpr uint32_t CU = PL ? 4 : (GRID ? RB : 1);
+      const unsigned char* const s_winb =
+          reinterpret_cast<const unsigned char*>(s_win) + (ONE && one >= 0 ? 4 * w_at(0, one) : 0);
+      auto gather4 = [&](auto N, uint2 c, const VT* v, VT* ak, VT* ak2) {
+        const uint32_t cc[4] = {c.x & 0xffffu, c.x >> 16, c.y & 0xffffu, c.y >> 16};
+        if constexpr (PL) {
+          constexpr int n = decltype(N)::value;
+          VT u[4][n];
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int s = 0; s < n; s++)
+              u[k][s] = reinterpret_cast<const VT*>(s_winb + cc[k] * CU)[32 * s];
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            VT* const y = (k & 1) ? ak2 : ak;
+            if constexpr (n >= 2) axpy_row<VT, 2>(v[k], u[k], y);
+            if constexpr (n == 4) axpy_row<VT, 2>(v[k], u[k] + 2, y + 2);
+            if constexpr (n & 1) y[n - 1] += v[k] * u[k][n - 1];
+          }
+        } else {
+          VT u[4][LD];
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            lds_row<VT, LD>(reinterpret_cast<const VT*>(s_winb + cc[k] * CU), 0, u[k]);
+          axpy_row<VT, LD>(v[0], u[0], ak);
+          axpy_row<VT, LD>(v[1], u[1], ak2);
+          axpy_row<VT, LD>(v[2], u[2], ak);
+          axpy_row<VT, LD>(v[3], u[3], ak2);
+        }
       };
-      auto row_done = [&](int sl, const VT ak[LD], const VT ak2[LD]) {
+      auto row_done = [&](auto N, int sl, const VT* ak, const VT* ak2) {
         const int lr = sl * 32 + lane;
-        if (lr < nrows) {
+        if (lr >= nrows) return;
+        if constexpr (ONE && decltype(N)::value == 1) {
+          const int at = w_at(lr, one);
+          const VT ur = s_win[at];
+          VT dg = VT(0);
+          if (o_diag >= 0)
+            dg = reinterpret_cast<const VT*>(s_dyn + o_diag)[at];
+          else if (a.diag)
+            dg = a.diag[(row0 + lr) * LD + one];
+          const VT wv = VT(a.A64.dscale[one]) * (ak[0] + ak2[0]) + dg * ur;
+          wu[0] += (double)wv * (double)ur;
+          s_w[at] = wv;
+        } else {
           VT ur[LD], dg[LD], wv[LD];
-          lds_row<VT, LD>(s_win, lr, ur);
+          w_ld(s_win, lr, ur);
           if (o_diag >= 0) {
-            lds_row<VT, LD>(reinterpret_cast<const VT*>(s_dyn + o_diag), lr, dg);
+            w_ld(reinterpret_cast<const VT*>(s_dyn + o_diag), lr, dg);
           } else {
 #pragma unroll
             for (int s = 0; s < LD; s++) dg[s] = VT(0);
             if (a.diag) ldv<VT, LD>(a.diag, row0 + lr, dg);
           }
 #pragma unroll
-          for (int s = 0; s < LD; s++) {
+          for (int s = 0; s < (PL ? NC : LD); s++) {
             wv[s] = VT(a.A64.dscale[s]) * (ak[s] + ak2[s]) + dg[s] * ur[s];
             if (s < NC) wu[s] += (double)wv[s] * (double)ur[s];
           }
-          sts_row<VT, LD>(s_w, lr, wv);
+          w_st(s_w, lr, wv);
         }
       };
       // slices in tensor memory: NS of the warp side by side (their loads and gathers
       // overlap); SC: columns in shared memory
-      auto tm_slices = [&](auto NSC, auto SC, int i, int sl) {
+      auto tm_slices = [&](auto N, auto NSC, auto SC, int i, int sl) {
+        constexpr int n = PL ? decltype(N)::value : LD;
         constexpr int NS = decltype(NSC)::value;
         constexpr int NG = 4 / VW;  // chunks of 4 entries per 16 tensor-memory columns
-        VT ak[NS][LD], ak2[NS][LD];
+        VT ak[NS][n], ak2[NS][n];
 #pragma unroll
         for (int j = 0; j < NS; j++)
 #pragma unroll
-          for (int s = 0; s < LD; s++) ak[j][s] = ak2[j][s] = VT(0);
+          for (int s = 0; s < n; s++) ak[j][s] = ak2[j][s] = VT(0);
 #pragma unroll
         for (int h = 0; h < VW; h++) {
           uint32_t tv[NS][16];
@@ -874,60 +1123,72 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
             VT v[4 * NG];
             memcpy(v, tv[j], sizeof(v));
 #pragma unroll
-            for (int g = 0; g < NG; g++) gather4(c[j][g], v + 4 * g, ak[j], ak2[j]);
+            for (int g = 0; g < NG; g++) gather4(N, c[j][g], v + 4 * g, ak[j], ak2[j]);
           }
         }
 #pragma unroll
-        for (int j = 0; j < NS; j++) row_done(sl + j * CC_W, ak[j], ak2[j]);
+        for (int j = 0; j < NS; j++) row_done(N, sl + j * CC_W, ak[j], ak2[j]);
       };
       // two where the rows' vectors leave the registers
-      constexpr int NS2 = RB <= 8 && RPT <= 2 ? 2 : 1;
-      int i = 0, sl = warp;
-      if (o_col >= 0) {
-        if constexpr (NS2 > 1) {
+      constexpr int NS2 = (PL && NC == 3) || (RB <= 8 && RPT <= 2) ? 2 : 1;
+      auto product = [&](auto N) {
+        int i = 0, sl = warp;
+        if (o_col >= 0) {
+          if constexpr (NS2 > 1) {
 #pragma unroll 1
-          for (; sl + CC_W < part.val_slice; i += 2, sl += 2 * CC_W)
-            tm_slices(std::integral_constant<int, NS2>{}, std::true_type{}, i, sl);
-        }
-#pragma unroll 1
-        for (; sl < part.val_slice; i++, sl += CC_W)
-          tm_slices(std::integral_constant<int, 1>{}, std::true_type{}, i, sl);
-      } else {
-#pragma unroll 1
-        for (; sl < part.val_slice; i++, sl += CC_W)
-          tm_slices(std::integral_constant<int, 1>{}, std::false_type{}, i, sl);
-      }
-#pragma unroll 1
-      for (; sl < part.nslices; sl += CC_W) {
-        const int base = s_sl[sl], nc = (s_sl[sl + 1] - base) >> 7;  // chunks of 4 entries
-        VT ak[LD], ak2[LD];
-#pragma unroll
-        for (int s = 0; s < LD; s++) ak[s] = ak2[s] = VT(0);
-#pragma unroll 4
-        for (int g = 0; g < nc; g++) {
-          const int e = base + 4 * lane + 128 * g;
-          VT v[4];
-          if (o_val >= 0) {
-            memcpy(v, __builtin_assume_aligned(s_val + (e - v0), 16), sizeof(v));
-          } else {
-#pragma unroll
-            for (int k = 0; k < VW; k++) {
-              const uint4 t = __ldcg(reinterpret_cast<const uint4*>(g_val + e) + k);
-              memcpy(reinterpret_cast<char*>(v) + 16 * k, &t, 16);
-            }
+            for (; sl + CC_W < part.val_slice; i += 2, sl += 2 * CC_W)
+              tm_slices(N, std::integral_constant<int, NS2>{}, std::true_type{}, i, sl);
           }
-          const uint2 c = o_col >= 0 ? *reinterpret_cast<const uint2*>(s_dyn + o_col + 2 * e)
-                                     : __ldg(reinterpret_cast<const uint2*>(g_col + e));
-          gather4(c, v, ak, ak2);
+#pragma unroll 1
+          for (; sl < part.val_slice; i++, sl += CC_W)
+            tm_slices(N, std::integral_constant<int, 1>{}, std::true_type{}, i, sl);
+        } else {
+#pragma unroll 1
+          for (; sl < part.val_slice; i++, sl += CC_W)
+            tm_slices(N, std::integral_constant<int, 1>{}, std::false_type{}, i, sl);
         }
-        row_done(sl, ak, ak2);
-      }
+#pragma unroll 1
+        for (; sl < part.nslices; sl += CC_W) {
+          const int base = s_sl[sl], nc = (s_sl[sl + 1] - base) >> 7;  // chunks of 4 entries
+          constexpr int n = PL ? decltype(N)::value : LD;
+          VT ak[n], ak2[n];
+#pragma unroll
+          for (int s = 0; s < n; s++) ak[s] = ak2[s] = VT(0);
+#pragma unroll 4
+          for (int g = 0; g < nc; g++) {
+            const int e = base + 4 * lane + 128 * g;
+            VT v[4];
+            if (o_val >= 0) {
+              memcpy(v, __builtin_assume_aligned(s_val + (e - v0), 16), sizeof(v));
+            } else {
+#pragma unroll
+              for (int k = 0; k < VW; k++) {
+                const uint4 t = __ldcg(reinterpret_cast<const uint4*>(g_val + e) + k);
+                memcpy(reinterpret_cast<char*>(v) + 16 * k, &t, 16);
+              }
+            }
+            const uint2 c = o_col >= 0 ? *reinterpret_cast<const uint2*>(s_dyn + o_col + 2 * e)
+                                       : __ldg(reinterpret_cast<const uint2*>(g_col + e));
+            gather4(N, c, v, ak, ak2);
+          }
+          row_done(N, sl, ak, ak2);
+        }
+      };
+      if (ONE && one >= 0)
+        product(std::integral_constant<int, 1>{});
+      else
+        product(std::integral_constant<int, NC>{});
 
       // ---- sums over the CTA, then to every CTA of the cluster
       {
-        const double v = WarpReduce<NC>::run(wu, lane);
-        const int id = WarpReduce<NC>::value_of(lane);
-        if (id >= 0) s_red[warp][8 + id] = v;
+        if (ONE && one >= 0) {
+          const double v = warp_sum(wu[0]);
+          if (lane == 0) s_red[warp][8 + one] = v;
+        } else {
+          const double v = WarpReduce<NC>::run(wu, lane);
+          const int id = WarpReduce<NC>::value_of(lane);
+          if (id >= 0) s_red[warp][8 + id] = v;
+        }
         __syncthreads();
         // a CTA that gave up sends no sums, so no other completes this pass either
         if (s_gave_up) {
@@ -936,7 +1197,8 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         }
         const int slot = tid & 15;
         const uint32_t dst = (uint32_t)(tid >> 4);
-        const bool used = (slot & 3) < NC && (slot < 12 || first);
+        const bool used = ONE && one >= 0 ? (slot & 3) == one && slot < 12
+                                         : (slot & 3) < NC && (slot < 12 || first);
         if (GRID ? (dst == 0 && used) : (dst < C && used)) {
           double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -1027,7 +1289,11 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
             s_al[lane] = runs ? (VT)st_alpha : VT(0);
             s_be[lane] = runs ? (VT)st_beta : VT(0);
           }
-          if (lane == 0) s_ctl = 0;
+          const unsigned run = __ballot_sync(0xffffffffu, runs);
+          if (lane == 0) {
+            s_ctl = 0;
+            s_run = (int)run;
+          }
         } else {
         const bool fine = isfinite(gm) && isfinite(rr) && isfinite(dl);
         bool coef = false;  // this lane takes new coefficients
@@ -1123,9 +1389,11 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           s_al[lane] = go ? (VT)st_alpha : VT(0);
           s_be[lane] = go ? (VT)st_beta : VT(0);
         }
+        const unsigned run = __ballot_sync(0xffffffffu, go);
         if (lane == 0) {
           s_ctl = ctl;
           s_mask = (int)tr_mask;
+          s_run = (int)run;
         }
         }
       }
@@ -1143,6 +1411,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       refresh = (ctl & CTL_REFRESH) != 0;
       fin = (ctl & CTL_FIN) != 0;
       tr_mask = (unsigned)s_mask;
+      if constexpr (ONE) one = !refresh && __popc(s_run) == 1 ? __ffs(s_run) - 1 : -1;
     }
 
     if (rank == 0 && warp == 0) {
@@ -1207,7 +1476,7 @@ __global__ void k_ccg_slices(CcgPart* parts, const int32_t* __restrict__ indptr,
 // One block per part.  The halo as a bitmap over the system's rows (shared memory), so its
 // ascending order and every column's window slot come from popcounts.  FILL = false: the
 // halo size and, per rank, the halo positions where that rank's rows begin; window-local
-// columns (times rb).  FILL = true: the push entries (rank of this part, slot, source row)
+// columns (times rb; planes > 0: words of a window in that many planes).  FILL = true: the push entries (rank of this part, slot, source row)
 // into the producers' lists at push_at (per producer and consumer), or, when halo is given
 // (GRID), the halo's rows at the part's push_off.
 template <bool FILL>
@@ -1215,7 +1484,7 @@ __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sy
                            const int32_t* __restrict__ sys_rows,
                            const int32_t* __restrict__ indptr,
                            const int32_t* __restrict__ indices,
-                           const int32_t* __restrict__ slices, int rb,
+                           const int32_t* __restrict__ slices, int rb, int planes,
                            uint16_t* __restrict__ loc_col,
                            int32_t* __restrict__ bounds, const int32_t* __restrict__ push_at,
                            uint32_t* __restrict__ push, int32_t* __restrict__ halo,
@@ -1291,7 +1560,8 @@ __global__ void k_ccg_halo(CcgPart* parts, int C, const int32_t* __restrict__ sy
           if (j >= 0 && j < n)
             c = (j >= own0 && j < own1) ? j - own0 : p.nrows + halo_pos(j);
         }
-        loc_col[p.entry_off + b + 128 * (k >> 2) + 4 * lane + (k & 3)] = (uint16_t)(c * rb);
+        loc_col[p.entry_off + b + 128 * (k >> 2) + 4 * lane + (k & 3)] = 
+            (uint16_t)(planes ? (c >> 5) * 32 * planes + (c & 31) : c * rb);
       }
     }
   } else {
@@ -1374,8 +1644,8 @@ struct Rpt {
   static constexpr int words = NC * (int)sizeof(VT) / 4;
   static constexpr int big = words == 1   ? 9
                              : words == 2 ? 6
-                             : words == 3 ? (GRID ? 4 : 3)
-                             : words == 4 ? 3
+                             : cc_planes<VT>(NC, 4, GRID) ? 4
+                             : words <= 4 ? 3
                                           : 2;
   static constexpr int small = GRID ? (words <= 2 ? 4 : (words <= 4 ? 2 : 1)) : (words <= 2 ? 2 : 1);
 };
@@ -1491,7 +1761,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   const tp_csr_op* op = ca.op;
   cudaStream_t st = ca.st;
   const int nsys = (int)sys.size(), ld = op->ld;
-  const size_t vt = inner_fp32 ? 4 : 8, rb = vt * ld;
+  const size_t vt = inner_fp32 ? 4 : 8;
   const int64_t most = rows[sys[0]];
   int dev = 0, optin = 0, big = 0;
   TP_CUDA_TRY(cudaGetDevice(&dev));
@@ -1499,6 +1769,10 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   const int rpt = rows_per_thread(most, C);
   void* fn = pick_kernel(inner_fp32 != 0, grid, ld, op->S, rpt, &big);
   if (rpt > big || rpt * CC_T > (1 << CC_SRC_BITS)) return TP_OK;
+  // columns of a window in planes, 0: rows of ld values
+  const int nc = ld < 4 ? ld : (op->S <= 3 ? 3 : 4);
+  const int planes = inner_fp32 && cc_planes<float>(nc, rpt, grid) ? nc : 0;
+  const size_t rb = planes ? 4 * (size_t)planes : vt * ld;
   cudaFuncAttributes fa;
   TP_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
   const size_t dyn = ((size_t)optin - fa.sharedSizeBytes - 1024) & ~(size_t)15;
@@ -1575,7 +1849,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   }
   const int unit = grid ? 1 : (int)rb;  // columns: window entries, or byte offsets
   k_ccg_halo<false><<<np, 512, bits, st>>>(h->d_parts, C, t_row0, t_rows, op->indptr,
-                                           op->indices, h->d_slices, unit, h->d_cols,
+                                           op->indices, h->d_slices, unit, planes, h->d_cols,
                                            grid ? nullptr : t_bounds, nullptr, nullptr, nullptr,
                                            t_flag);
   TP_LAUNCH_CHECK();
@@ -1606,9 +1880,9 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
       p.npush = (int32_t)(npush - p.push_off);
       win_cap = std::max(win_cap, p.nrows + p.nhalo);
     }
-  win_cap = (win_cap + 3) & ~3;
+  win_cap = (win_cap + 31) & ~31;
   // window columns are 16-bit
-  if (npush > INT32_MAX || win_cap * unit > 65536) return TP_OK;
+  if (npush > INT32_MAX || win_cap * (planes ? planes : unit) > 65536) return TP_OK;
   if (!grid && win_cap >= (1 << CC_SLOT_BITS)) return TP_OK;
   // what has to fit in shared memory (the kernel carves in the same order); columns and
   // values stream from L2 where they do not
@@ -1616,9 +1890,10 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
   for (const CcgPart& p : parts) {
     auto r16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
     size_t need = 2 * 16 * 16 * sizeof(double) + rb * (size_t)win_cap;
-    need += r16(rb * (size_t)p.nrows) + r16(4 * ((size_t)p.nslices + 1)) + r16(4 * (size_t)p.npush);
+    const size_t own = rb * (size_t)(planes ? 32 * p.nslices : p.nrows);
+    need += r16(own) + r16(4 * ((size_t)p.nslices + 1)) + r16(4 * (size_t)p.npush);
     if (need > dyn) return TP_OK;
-    if (op->diag64) need += r16(rb * (size_t)p.nrows);
+    if (op->diag64) need += r16(own);
     const size_t nval = (size_t)(p.entries - sl_host[p.slice_off + p.val_slice]);
     need += r16(2 * (size_t)p.entries) + r16(vt * nval);
     spill |= nval > 0 && need > dyn;
@@ -1654,7 +1929,7 @@ int build_class(CcgClass* h, const CreateArgs& ca, int inner_fp32, const std::ve
     TP_CUDA_TRY(cudaMemcpyAsync(t_at, at.data(), sizeof(int32_t) * n_at, cudaMemcpyHostToDevice,
                                 st));
   k_ccg_halo<true><<<np, 512, bits, st>>>(h->d_parts, C, t_row0, t_rows, op->indptr,
-                                          op->indices, h->d_slices, unit, h->d_cols, t_bounds,
+                                          op->indices, h->d_slices, unit, planes, h->d_cols, t_bounds,
                                           t_at, h->d_push, grid ? h->d_halo : nullptr, t_flag);
   TP_LAUNCH_CHECK();
   TP_CUDA_TRY(cudaStreamSynchronize(st));

@@ -59,7 +59,8 @@ def _check(op, sol, res, b, rtol):
     (27, 4, True, False, "exchange"), (28, 2, False, False, "exchange"),
     (24, 3, False, False, "exchange"), (22, 4, False, True, "exchange"),
     (34, 2, True, False, "exchange"), (48, 1, False, False, "exchange"),
-    (44, 3, True, False, "exchange")])
+    (44, 3, True, False, "exchange"), (55, 3, True, True, "exchange"),
+    (56, 3, True, False, "exchange"), (54, 4, True, True, "exchange")])
 def test_engine_matches_grid_engine(cuda_device, monkeypatch, n, S, fp32, bc, engine):
     import torch
     from dissolve_tp.krylov import PersistentCG
