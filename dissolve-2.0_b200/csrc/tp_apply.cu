@@ -1,47 +1,64 @@
 // tp_apply.cu -- matrix-free operator apply and the standalone multi-column CSR apply.
 //
 // Matrix-free (replaces gpu/ceed_operators.py CeedDiffusionMassOp / DiffMassBilinear,
-// :87-108, 247-353): one thread per cell gathers its 4 vertex coordinates with
-// 32-byte loads, recomputes J, det J and the cofactor rows c_k = (J^-1 row k) det J in
-// FP64, and applies, for every column s,
-//     y_i += scale (c_i . w) + react M_e u,    w = sum_k (u_k - u_0) c_k
-// with scale = De/(6|det J|) (exact P1 stiffness) or 4 De/det^2 (legacy: the reference
-// QFunction drops wdetJ), and consistent (|det|/120 (1+d_ij)) or lumped (|det|/24) mass.
+// :87-108, 247-353): one thread per cell takes the cell's geometry record (G = J^-1 J^-T and
+// |det J|, 64 bytes) and applies, for every column s,
+//     y_i += scale (G d)_i + react M_e u,    d_k = u_k - u_0,   y_0 += -(sum of the others)
+// with scale = De |det J|/6 (exact P1 stiffness) or 4 De (legacy: the reference QFunction
+// drops wdetJ), and consistent (|det|/120 (1+d_ij)) or lumped (|det|/24) mass.  A mesh
+// without geometry records gathers its 4 vertex coordinates with 32-byte loads and
+// recomputes J, det J and the cofactor rows c_k = (J^-1 row k) det J in FP64 instead:
+// y_i += scale (c_i . w), w = sum_k d_k c_k, scale = De/(6|det J|) or 4 De/det^2.
 // Contributions land with hardware atomics (FP32 columns as one 16-byte vector atomic),
 // so the result's last bits depend on arrival order, as in the reference.  A warp takes
 // 32 consecutive cells.  Scalar atomics (FP64, FP32 rows narrower than 16 bytes) are
 // grouped: for each local vertex slot, a run of consecutive lanes whose cells have the
-// same vertex in that slot sums its contributions through shared memory and the run's
-// first lane issues the atomics.  The six cells of a Kuhn cube share their first and last
+// same vertex in that slot sums its contributions by doubling and the run's first lane
+// issues the atomics.  The six cells of a Kuhn cube share their first and last
 // vertex (runs of six) and pairs of them their second (runs of two): 11 atomics per cube
 // instead of 24; on any other ordering the runs are single lanes.  A 16-byte FP32 row
 // goes out as one vector atomic per lane, where the grouping does not pay.
+//
+// Bound by latency and by the L1's handling of gathers and atomics, not by memory: the
+// records cost 56 bytes per cell more than the coordinates but half the gathers, no
+// division and 20 registers; the vertices of a thread's next cell are loaded a turn ahead,
+// so a turn waits for memory once; the grid is what is resident (4 blocks an SM: 44.0 us a
+// call, 3 or twice as many blocks than resident 46 to 48).  1,572,864 cells, one FP64
+// column: 46.7 us from coordinates, 39.1 from records, 31.0 with the loads ahead and the
+// runs summed by shuffles instead of through shared memory.
 #include "tp_ops.cuh"
 
 namespace tp {
 
-// CS columns of LD are used (compile time, so the column loops carry no predicates).
-template <typename T, int LD, int CS>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_matfree(
+// CS columns of LD are used (compile time, so the column loops carry no predicates).  GEO:
+// geometry records, else coordinates.  Blocks per SM: 4 where their 64 registers hold a cell
+// (three FP64 columns of 1,572,864 cells: 71.4 us with 4, 64.2 with 3; 68.4 before records).
+constexpr int mf_blocks(bool geo, size_t value, int cs) {
+  return value == 4 || (geo && cs < 3) ? 4 : 3;
+}
+template <typename T, int LD, int CS, bool GEO>
+__global__ void __launch_bounds__(256, mf_blocks(GEO, sizeof(T), CS)) k_matfree(
     int64_t n, const int4* __restrict__ cells, const double4* __restrict__ X,
-    const double* __restrict__ De, const double* __restrict__ alpha, double4 dsc, double4 shf,
-    double inv_dt, int lumped, int legacy, const T* __restrict__ x, T* __restrict__ y) {
+    const double* __restrict__ geo, const double* __restrict__ De,
+    const double* __restrict__ alpha, double4 dsc, double4 shf, double inv_dt, int lumped,
+    int legacy, const T* __restrict__ x, T* __restrict__ y) {
   constexpr bool VEC = sizeof(T) == 4 && LD == 4;  // one 16-byte vector atomic per row
   constexpr int WPB = 256 / 32;
-  __shared__ T s_val[VEC ? 1 : WPB][32][CS];  // one contribution per lane, for the run head
   const double dscale[4] = {dsc.x, dsc.y, dsc.z, dsc.w};
   const double shift[4] = {shf.x, shf.y, shf.z, shf.w};
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t wstride = (int64_t)gridDim.x * WPB * 32;
   // the loop trip count is uniform over the warp: lanes past n compute a copy of the
   // last cell and add nothing
-  for (int64_t base = ((int64_t)blockIdx.x * WPB + wib) * 32; base < n; base += wstride) {
+  const int64_t base0 = ((int64_t)blockIdx.x * WPB + wib) * 32;
+  int4 vn = make_int4(0, 0, 0, 0);  // the next turn's vertices: their loads lead the others
+  if (base0 < n) vn = cells[min(base0 + lane, n - 1)];
+  for (int64_t base = base0; base < n; base += wstride) {
     const int64_t c0 = base + lane;
     const bool valid = c0 < n;
     const int64_t c = valid ? c0 : n - 1;
-    const int4 v = cells[c];
-    const double4 x0 = ldg_d4(X + v.x), x1 = ldg_d4(X + v.y), x2 = ldg_d4(X + v.z),
-                  x3 = ldg_d4(X + v.w);
+    const int4 v = vn;
+    if (base + wstride < n) vn = cells[min(c0 + wstride, n - 1)];
     T xv[4][LD];
     ldv<T, LD>(x, v.x, xv[0]);
     ldv<T, LD>(x, v.y, xv[1]);
@@ -49,29 +66,46 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_matfree(
     ldv<T, LD>(x, v.w, xv[3]);
     const double De_c = De[c];
     const double al = alpha ? alpha[c] : 0.0;
-    const double e[3][3] = {{x1.x - x0.x, x1.y - x0.y, x1.z - x0.z},
-                            {x2.x - x0.x, x2.y - x0.y, x2.z - x0.z},
-                            {x3.x - x0.x, x3.y - x0.y, x3.z - x0.z}};
-    double cr[3][3];  // cr[k] = row k of adj(J): e2 x e3, e3 x e1, e1 x e2
-    cr[0][0] = e[1][1] * e[2][2] - e[1][2] * e[2][1];
-    cr[0][1] = e[1][2] * e[2][0] - e[1][0] * e[2][2];
-    cr[0][2] = e[1][0] * e[2][1] - e[1][1] * e[2][0];
-    cr[1][0] = e[2][1] * e[0][2] - e[2][2] * e[0][1];
-    cr[1][1] = e[2][2] * e[0][0] - e[2][0] * e[0][2];
-    cr[1][2] = e[2][0] * e[0][1] - e[2][1] * e[0][0];
-    cr[2][0] = e[0][1] * e[1][2] - e[0][2] * e[1][1];
-    cr[2][1] = e[0][2] * e[1][0] - e[0][0] * e[1][2];
-    cr[2][2] = e[0][0] * e[1][1] - e[0][1] * e[1][0];
-    const double det = e[0][0] * cr[0][0] + e[0][1] * cr[0][1] + e[0][2] * cr[0][2];
-    const double adet = fabs(det);
-    // one division: De/(6|det|), or 4 De/det^2 for the legacy QFunction
-    const double kbase = legacy ? (4.0 * De_c) / (det * det) : De_c / (6.0 * adet);
-    const double mbase = adet * (lumped ? 1.0 / 24.0 : 1.0 / 120.0);
+    // c_: G, or the cofactor rows
+    double adet, kbase;
     T c_[3][3];
+    if constexpr (GEO) {
+      const double4* gp = reinterpret_cast<const double4*>(geo) + 2 * c;
+      const double4 g0 = ldg_d4(gp), g1 = ldg_d4(gp + 1);
+      adet = g1.z;
+      kbase = legacy ? 4.0 * De_c : De_c * adet * (1.0 / 6.0);
+      c_[0][0] = (T)g0.x;
+      c_[0][1] = c_[1][0] = (T)g0.y;
+      c_[0][2] = c_[2][0] = (T)g0.z;
+      c_[1][1] = (T)g0.w;
+      c_[1][2] = c_[2][1] = (T)g1.x;
+      c_[2][2] = (T)g1.y;
+    } else {
+      const double4 x0 = ldg_d4(X + v.x), x1 = ldg_d4(X + v.y), x2 = ldg_d4(X + v.z),
+                    x3 = ldg_d4(X + v.w);
+      const double e[3][3] = {{x1.x - x0.x, x1.y - x0.y, x1.z - x0.z},
+                              {x2.x - x0.x, x2.y - x0.y, x2.z - x0.z},
+                              {x3.x - x0.x, x3.y - x0.y, x3.z - x0.z}};
+      double cr[3][3];  // cr[k] = row k of adj(J): e2 x e3, e3 x e1, e1 x e2
+      cr[0][0] = e[1][1] * e[2][2] - e[1][2] * e[2][1];
+      cr[0][1] = e[1][2] * e[2][0] - e[1][0] * e[2][2];
+      cr[0][2] = e[1][0] * e[2][1] - e[1][1] * e[2][0];
+      cr[1][0] = e[2][1] * e[0][2] - e[2][2] * e[0][1];
+      cr[1][1] = e[2][2] * e[0][0] - e[2][0] * e[0][2];
+      cr[1][2] = e[2][0] * e[0][1] - e[2][1] * e[0][0];
+      cr[2][0] = e[0][1] * e[1][2] - e[0][2] * e[1][1];
+      cr[2][1] = e[0][2] * e[1][0] - e[0][0] * e[1][2];
+      cr[2][2] = e[0][0] * e[1][1] - e[0][1] * e[1][0];
+      const double det = e[0][0] * cr[0][0] + e[0][1] * cr[0][1] + e[0][2] * cr[0][2];
+      adet = fabs(det);
+      // one division: De/(6|det|), or 4 De/det^2 for the legacy QFunction
+      kbase = legacy ? (4.0 * De_c) / (det * det) : De_c / (6.0 * adet);
 #pragma unroll
-    for (int a = 0; a < 3; a++)
+      for (int a = 0; a < 3; a++)
 #pragma unroll
-      for (int b = 0; b < 3; b++) c_[a][b] = (T)cr[a][b];
+        for (int b = 0; b < 3; b++) c_[a][b] = (T)cr[a][b];
+    }
+    const double mbase = adet * (lumped ? 1.0 / 24.0 : 1.0 / 120.0);
     T out[4][CS];
 #pragma unroll
     for (int s = 0; s < CS; s++) {
@@ -84,7 +118,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_matfree(
       T yk[4];
 #pragma unroll
       for (int i = 1; i < 4; i++)
-        yk[i] = ks * (c_[i - 1][0] * w[0] + c_[i - 1][1] * w[1] + c_[i - 1][2] * w[2]);
+        yk[i] = GEO ? ks * w[i - 1]
+                    : ks * (c_[i - 1][0] * w[0] + c_[i - 1][1] * w[1] + c_[i - 1][2] * w[2]);
       yk[0] = -(yk[1] + yk[2] + yk[3]);
       if (lumped) {
 #pragma unroll
@@ -116,23 +151,19 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_matfree(
       const bool head = lane == 0 || prev != key;
       const unsigned above = (__ballot_sync(0xffffffffu, head) >> lane) >> 1;
       const int end = above ? lane + __ffs(above) : 32;  // run = lanes [lane, end)
-      if (!head) {
+      // sums of the runs by doubling: after step d a lane holds the sum of its next 2 d lanes
+      const int longest = __reduce_max_sync(0xffffffffu, end - lane);
+      for (int d = 1; d < longest; d *= 2) {
 #pragma unroll
-        for (int s = 0; s < CS; s++) s_val[wib][lane][s] = out[i][s];
-      }
-      __syncwarp();
-      if (head && valid) {
-        T acc[CS];
-#pragma unroll
-        for (int s = 0; s < CS; s++) acc[s] = out[i][s];
-        for (int l = lane + 1; l < end; l++) {
-#pragma unroll
-          for (int s = 0; s < CS; s++) acc[s] += s_val[wib][l][s];
+        for (int s = 0; s < CS; s++) {
+          const T t = __shfl_down_sync(0xffffffffu, out[i][s], d);
+          if (lane + d < end) out[i][s] += t;
         }
-#pragma unroll
-        for (int s = 0; s < CS; s++) atomicAdd(dst + s, acc[s]);
       }
-      __syncwarp();
+      if (head && valid) {
+#pragma unroll
+        for (int s = 0; s < CS; s++) atomicAdd(dst + s, out[i][s]);
+      }
     }
   }
 }
@@ -514,11 +545,18 @@ template <typename T, int LD, int CS>
 static void launch_matfree_cs(const tp_mesh* m, const double* De, const double* al, double4 dsc,
                               double4 shf, double inv_dt, int lumped, int legacy, const void* x,
                               void* y, cudaStream_t st) {
-  const int grid = grid_for(m->n_cells, 256, sm_count() * 8);
-  k_matfree<T, LD, CS><<<grid, 256, 0, st>>>(
-      m->n_cells, reinterpret_cast<const int4*>(m->cells),
-      reinterpret_cast<const double4*>(m->coords4), De, al, dsc, shf, inv_dt, lumped, legacy,
-      static_cast<const T*>(x), static_cast<T*>(y));
+  auto launch = [&](auto geo) {
+    const int grid = grid_for(m->n_cells, 256,
+                              sm_count() * mf_blocks(decltype(geo)::value, sizeof(T), CS));
+    k_matfree<T, LD, CS, decltype(geo)::value><<<grid, 256, 0, st>>>(
+        m->n_cells, reinterpret_cast<const int4*>(m->cells),
+        reinterpret_cast<const double4*>(m->coords4), m->geo, De, al, dsc, shf, inv_dt, lumped,
+        legacy, static_cast<const T*>(x), static_cast<T*>(y));
+  };
+  if (m->geo && (reinterpret_cast<uintptr_t>(m->geo) & 31) == 0)
+    launch(std::true_type{});
+  else
+    launch(std::false_type{});
 }
 
 template <typename T>

@@ -321,7 +321,8 @@ TP_API int tp_unpack_columns(int64_t n, int S, int ld, const double* src, double
 /* ------------------------------------------------------------------ operators */
 /* gpu/ceed_operators.py:87-108, 247-353 as intended, on S interleaved columns:
  * y[:, s] = sum_e [diff_scale[s] De_e K_e + (inv_dt + alpha_e + shift[s]) M_e] x_e[:, s]
- * recomputing the P1 gradients of every cell from coords4 in FP64.  legacy != 0 weights
+ * from the geometry records (m->geo), or with geo NULL recomputing the P1 gradients of every
+ * cell from coords4 in FP64; coords4 is required either way.  legacy != 0 weights
  * the stiffness by 4 (the reference QFunction omits wdetJ, :101-104) instead of |detJ|/6.
  * fp32 != 0: x, y float (geometry still FP64).  diff_scale/shift: host, S values, or NULL.
  * y is overwritten. */
