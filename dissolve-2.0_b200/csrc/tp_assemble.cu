@@ -767,65 +767,165 @@ __global__ void k_rhs_bc(int64_t n_bc, const int32_t* __restrict__ bc, int64_t n
   for (int s = 0; s < S; s++) b[v0 * ld + s] = v[s];
 }
 
+// ----------------------------------------------------------------- ordered sums over tiles
+// Sums over a row's cells of N values that depend on the cell alone.  A tile's cells compute
+// theirs once into shared memory (N planes, the last slot zero for the padding terms); then
+// a thread per row and value adds the row's terms in ascending cell order, 8 at a time: the
+// sums of the row walks, bit for bit, with each cell's arithmetic and loads done by about 1.7
+// tiles instead of by all 4 of its rows, which walked them one cell's latency at a time.
+// out(row, n, sum) is called by whole warps, N consecutive lanes per row (row < 0: none).
+// Bound by the L1's gathers of the cells' data and the shared-memory reads of the terms;
+// BLOCKS per SM as measured (more until the registers spill; several cells of a thread side
+// by side take longer).  274,625 vertices, us in a row walk and on tiles: gradient 138 and
+// 76, lumped diagonal of three columns with reaction 101 and 58, of one 43 and 29; 4,913
+// vertices 21 and 8, 13 and 6, 8 and 5.
+template <int N, int BLOCKS, class Cell, class Out>
+__global__ void __launch_bounds__(256, BLOCKS) k_cell_sums_tiles(TileView tv, Cell cell, Out out) {
+  extern __shared__ double s_cs[];
+  constexpr int T = 256;
+  const int R = tv.R, t = blockIdx.x, tid = threadIdx.x;
+  const TileHead h = tile_head(tv, t);
+  const int m = h.m, M = m + 1;
+  constexpr int MAXC = 4;
+  int32_t cid[MAXC];
+#pragma unroll
+  for (int k = 0; k < MAXC; k++) {
+    const int i = tid + k * T;
+    cid[k] = (i < m) ? __ldg(tv.cells + h.c0 + i) : -1;
+  }
+  auto put = [&](int i, int64_t c) {
+    double v[N];
+    cell(c, v);
+#pragma unroll
+    for (int n = 0; n < N; n++) s_cs[n * M + i] = v[n];
+  };
+#pragma unroll
+  for (int k = 0; k < MAXC; k++)
+    if (cid[k] >= 0) put(tid + k * T, cid[k]);
+  for (int i = tid + MAXC * T; i < m; i += T) put(i, __ldg(tv.cells + h.c0 + i));
+  if (tid < N) s_cs[tid * M + m] = 0.0;
+  __syncthreads();
+  const int rows = (R * N + T - 1) / T * T;  // whole warps
+  for (int q = tid; q < rows; q += T) {
+    const int lr = q / N, n = q % N;
+    const int64_t r = lr < R ? __ldg(tv.rows + (int64_t)t * R + lr) : -1;
+    double acc = 0.0;
+    if (r >= 0) {
+      const uint4* const dv = reinterpret_cast<const uint4*>(tv.dterms + h.d0 + (int64_t)lr * h.KD);
+      const double* const sv = s_cs + n * M;
+      for (int g = 0; 8 * g < h.KD; g++) {
+        const uint4 g8 = __ldg(dv + g);
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = sv[term_of(g8, k) & TILE_LOC_MASK];
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc = __dadd_rn(acc, v[k]);
+      }
+    }
+    out(r, n, acc);
+  }
+}
+
+// the lumped diagonal's terms, as in k_lumped_diag
+template <int N>
+struct LumpedDiagCell {
+  int S, ld;
+  const double* geo;
+  const double* alpha;
+  double4 shift;
+  __device__ void operator()(int64_t c, double v[N]) const {
+    const double sh[4] = {shift.x, shift.y, shift.z, shift.w};
+    const double Ld = __dmul_rn(div120(__ldg(geo + 8 * c + 6)), 5.0);
+#pragma unroll
+    for (int s = 0; s < N; s++)
+      v[s] = s < S ? __dmul_rn(__dadd_rn(sh[s], alpha ? __ldg(alpha + c * ld + s) : 0.0), Ld) : 0.0;
+  }
+};
+struct LumpedDiagOut {
+  int ld;
+  const uint8_t* bc_mask;
+  double* d64;
+  float* d32;
+  __device__ void operator()(int64_t r, int s, double sum) const {
+    if (r < 0 || s >= ld) return;
+    const double v = bc_mask && bc_mask[r] ? 1.0 : sum;
+    if (d64) d64[r * ld + s] = v;
+    if (d32) d32[r * ld + s] = (float)v;
+  }
+};
+
 // ----------------------------------------------------------------- nodal gradient
-// gpu_assembler.py:251-304 + :672, row-gathered
-__global__ void k_nodal_gradient(int64_t nv, const int32_t* __restrict__ cells,
-                                 const int32_t* __restrict__ v2c_ptr,
-                                 const int32_t* __restrict__ v2c, const double* __restrict__ geo,
-                                 const double* __restrict__ JinvT,
-                                 const double* __restrict__ coords4, const double* __restrict__ u,
+// gpu_assembler.py:251-304 + :672, row-gathered.  A cell's terms: volume times gradient, and
+// the volume.
+struct GradientCell {
+  const int4* cells;
+  const double* geo;
+  const double* JinvT;    // or
+  const double4* X;       // coordinates
+  const double* u;
+  __device__ void operator()(int64_t c, double v[4]) const {
+    const int4 cv = __ldg(cells + c);
+    const double u0 = __ldg(u + cv.x), u1 = __ldg(u + cv.y), u2 = __ldg(u + cv.z),
+                 u3 = __ldg(u + cv.w);
+    const double g0 = __dadd_rn(-u0, u1), g1 = __dadd_rn(-u0, u2), g2 = __dadd_rn(-u0, u3);
+    double JT[9];
+    if (JinvT) {
+#pragma unroll
+      for (int q = 0; q < 9; q++) JT[q] = __ldg(JinvT + 9 * c + q);
+    } else {
+      const double4 x0 = ldg_d4(X + cv.x), x1 = ldg_d4(X + cv.y), x2 = ldg_d4(X + cv.z),
+                    x3 = ldg_d4(X + cv.w);
+      const double e[3][3] = {{x1.x - x0.x, x1.y - x0.y, x1.z - x0.z},
+                              {x2.x - x0.x, x2.y - x0.y, x2.z - x0.z},
+                              {x3.x - x0.x, x3.y - x0.y, x3.z - x0.z}};
+      double cr[3][3];
+      cr[0][0] = e[1][1] * e[2][2] - e[1][2] * e[2][1];
+      cr[0][1] = e[1][2] * e[2][0] - e[1][0] * e[2][2];
+      cr[0][2] = e[1][0] * e[2][1] - e[1][1] * e[2][0];
+      cr[1][0] = e[2][1] * e[0][2] - e[2][2] * e[0][1];
+      cr[1][1] = e[2][2] * e[0][0] - e[2][0] * e[0][2];
+      cr[1][2] = e[2][0] * e[0][1] - e[2][1] * e[0][0];
+      cr[2][0] = e[0][1] * e[1][2] - e[0][2] * e[1][1];
+      cr[2][1] = e[0][2] * e[1][0] - e[0][0] * e[1][2];
+      cr[2][2] = e[0][0] * e[1][1] - e[0][1] * e[1][0];
+      const double inv =
+          1.0 / (e[0][0] * cr[0][0] + e[0][1] * cr[0][1] + e[0][2] * cr[0][2]);
+      // J^-T[a][b] = J^-1[b][a] = cr[b][a] / det
+#pragma unroll
+      for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int bb = 0; bb < 3; bb++) JT[3 * a + bb] = cr[bb][a] * inv;
+    }
+    const double w = div6(__ldg(geo + 8 * c + 6));
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      v[a] = __dmul_rn(w, __dadd_rn(__dadd_rn(__dmul_rn(JT[3 * a], g0), __dmul_rn(JT[3 * a + 1], g1)),
+                                    __dmul_rn(JT[3 * a + 2], g2)));
+    v[3] = w;
+  }
+};
+struct GradientOut {
+  double* grad;
+  __device__ void operator()(int64_t r, int n, double sum) const {
+    const double ws = __shfl_sync(0xffffffffu, sum, (threadIdx.x & 31) | 3);
+    if (r >= 0 && n < 3) grad[3 * r + n] = __ddiv_rn(sum, ws);
+  }
+};
+
+__global__ void k_nodal_gradient(int64_t nv, const int32_t* __restrict__ v2c_ptr,
+                                 const int32_t* __restrict__ v2c, GradientCell cell,
                                  double* __restrict__ grad) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nv;
        r += (int64_t)gridDim.x * blockDim.x) {
-    double gx = 0.0, gy = 0.0, gz = 0.0, ws = 0.0;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
     for (int k = v2c_ptr[r]; k < v2c_ptr[r + 1]; k++) {
-      const int64_t c = v2c[k] >> 2;
-      const int4 cv = reinterpret_cast<const int4*>(cells)[c];
-      const double u0 = u[cv.x], u1 = u[cv.y], u2 = u[cv.z], u3 = u[cv.w];
-      const double g0 = __dadd_rn(-u0, u1), g1 = __dadd_rn(-u0, u2), g2 = __dadd_rn(-u0, u3);
-      double JT[9];
-      if (JinvT) {
+      double v[4];
+      cell(v2c[k] >> 2, v);
 #pragma unroll
-        for (int q = 0; q < 9; q++) JT[q] = JinvT[9 * c + q];
-      } else {
-        const double4* X = reinterpret_cast<const double4*>(coords4);
-        const double4 x0 = X[cv.x], x1 = X[cv.y], x2 = X[cv.z], x3 = X[cv.w];
-        const double e[3][3] = {{x1.x - x0.x, x1.y - x0.y, x1.z - x0.z},
-                                {x2.x - x0.x, x2.y - x0.y, x2.z - x0.z},
-                                {x3.x - x0.x, x3.y - x0.y, x3.z - x0.z}};
-        double cr[3][3];
-        cr[0][0] = e[1][1] * e[2][2] - e[1][2] * e[2][1];
-        cr[0][1] = e[1][2] * e[2][0] - e[1][0] * e[2][2];
-        cr[0][2] = e[1][0] * e[2][1] - e[1][1] * e[2][0];
-        cr[1][0] = e[2][1] * e[0][2] - e[2][2] * e[0][1];
-        cr[1][1] = e[2][2] * e[0][0] - e[2][0] * e[0][2];
-        cr[1][2] = e[2][0] * e[0][1] - e[2][1] * e[0][0];
-        cr[2][0] = e[0][1] * e[1][2] - e[0][2] * e[1][1];
-        cr[2][1] = e[0][2] * e[1][0] - e[0][0] * e[1][2];
-        cr[2][2] = e[0][0] * e[1][1] - e[0][1] * e[1][0];
-        const double inv =
-            1.0 / (e[0][0] * cr[0][0] + e[0][1] * cr[0][1] + e[0][2] * cr[0][2]);
-        // J^-T[a][b] = J^-1[b][a] = cr[b][a] / det
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-          for (int bb = 0; bb < 3; bb++) JT[3 * a + bb] = cr[bb][a] * inv;
-      }
-      const double px = __dadd_rn(__dadd_rn(__dmul_rn(JT[0], g0), __dmul_rn(JT[1], g1)),
-                                  __dmul_rn(JT[2], g2));
-      const double py = __dadd_rn(__dadd_rn(__dmul_rn(JT[3], g0), __dmul_rn(JT[4], g1)),
-                                  __dmul_rn(JT[5], g2));
-      const double pz = __dadd_rn(__dadd_rn(__dmul_rn(JT[6], g0), __dmul_rn(JT[7], g1)),
-                                  __dmul_rn(JT[8], g2));
-      const double w = div6(geo[8 * c + 6]);
-      gx = __dadd_rn(gx, __dmul_rn(w, px));
-      gy = __dadd_rn(gy, __dmul_rn(w, py));
-      gz = __dadd_rn(gz, __dmul_rn(w, pz));
-      ws = __dadd_rn(ws, w);
+      for (int n = 0; n < 4; n++) s[n] = __dadd_rn(s[n], v[n]);
     }
-    grad[3 * r + 0] = __ddiv_rn(gx, ws);
-    grad[3 * r + 1] = __ddiv_rn(gy, ws);
-    grad[3 * r + 2] = __ddiv_rn(gz, ws);
+#pragma unroll
+    for (int n = 0; n < 3; n++) grad[3 * r + n] = __ddiv_rn(s[n], s[3]);
   }
 }
 
@@ -1259,6 +1359,14 @@ extern "C" int tp_dirichlet_rows(int64_t n_bc, const int32_t* bc_dofs, int64_t n
   return TP_OK;
 }
 
+// Shared memory of k_cell_sums_tiles for N values per cell, 0: no tiles, or tiles of so many
+// cells that the row walk is taken (more than 48 KB: fewer than 4 tiles would share an SM).
+static size_t cell_sums_smem(const tp_mesh* m, int N) {
+  if (!m->tiles || m->tiles->v.n_tiles <= 0) return 0;
+  const size_t smem = sizeof(double) * N * ((size_t)m->tiles->v.max_cells + 1);
+  return smem <= 48 * 1024 ? smem : 0;
+}
+
 extern "C" int tp_lumped_diag(const tp_mesh* m, int S, int ld, const double* alpha,
                               const double* shift, const uint8_t* bc_mask, double* diag64,
                               float* diag32, void* stream) {
@@ -1268,9 +1376,27 @@ extern "C" int tp_lumped_diag(const tp_mesh* m, int S, int ld, const double* alp
   double sh[4] = {0, 0, 0, 0};
   for (int s = 0; s < S; s++) sh[s] = shift ? shift[s] : 0.0;
   if (m->n_verts == 0) return TP_OK;
-  k_lumped_diag<<<grid_for(m->n_verts, 128, 65535), 128, 0, as_stream(stream)>>>(
-      m->n_verts, S, ld, m->v2c_ptr, m->v2c, m->geo, alpha, make_double4(sh[0], sh[1], sh[2], sh[3]),
-      bc_mask, diag64, diag32);
+  const double4 shf = make_double4(sh[0], sh[1], sh[2], sh[3]);
+  const int N = ld <= 2 ? ld : 4;
+  const size_t smem = cell_sums_smem(m, N);
+  if (smem) {
+    const TileView& tv = m->tiles->v;
+    const LumpedDiagOut out{ld, bc_mask, diag64, diag32};
+    auto run = [&](auto n) {
+      constexpr int NN = decltype(n)::value;
+      k_cell_sums_tiles<NN, NN == 4 ? 6 : 8><<<tv.n_tiles, 256, smem, as_stream(stream)>>>(
+          tv, LumpedDiagCell<NN>{S, ld, m->geo, alpha, shf}, out);
+    };
+    if (N == 1)
+      run(std::integral_constant<int, 1>{});
+    else if (N == 2)
+      run(std::integral_constant<int, 2>{});
+    else
+      run(std::integral_constant<int, 4>{});
+  } else {
+    k_lumped_diag<<<grid_for(m->n_verts, 128, 65535), 128, 0, as_stream(stream)>>>(
+        m->n_verts, S, ld, m->v2c_ptr, m->v2c, m->geo, alpha, shf, bc_mask, diag64, diag32);
+  }
   TP_LAUNCH_CHECK();
   return TP_OK;
 }
@@ -1376,8 +1502,16 @@ extern "C" int tp_nodal_gradient(const tp_mesh* m, const double* JinvT, const do
   TP_REQUIRE(mesh_ok(m) && u && grad, "null pointer");
   TP_REQUIRE(JinvT || m->coords4, "need JinvT or coords4");
   if (m->n_verts == 0) return TP_OK;
-  k_nodal_gradient<<<grid_for(m->n_verts, 128, 65535), 128, 0, as_stream(stream)>>>(
-      m->n_verts, m->cells, m->v2c_ptr, m->v2c, m->geo, JinvT, m->coords4, u, grad);
+  const GradientCell cell{reinterpret_cast<const int4*>(m->cells), m->geo, JinvT,
+                          reinterpret_cast<const double4*>(m->coords4), u};
+  const size_t smem = cell_sums_smem(m, 4);
+  if (smem) {
+    k_cell_sums_tiles<4, 5><<<m->tiles->v.n_tiles, 256, smem, as_stream(stream)>>>(
+        m->tiles->v, cell, GradientOut{grad});
+  } else {
+    k_nodal_gradient<<<grid_for(m->n_verts, 128, 65535), 128, 0, as_stream(stream)>>>(
+        m->n_verts, m->v2c_ptr, m->v2c, cell, grad);
+  }
   TP_LAUNCH_CHECK();
   return TP_OK;
 }

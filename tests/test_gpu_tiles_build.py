@@ -91,3 +91,47 @@ def test_tiles_assemble_like_the_row_walk(cuda_device, kind, rows):
     assert out[1][0] == -7.0 and out[1][-1] == -7.0  # nothing written outside the values
     info = dm.tiles_info()
     assert info["n_tiles"] == -(-dm.n_verts // rows)
+
+
+@pytest.mark.parametrize("rows", [32, 64, 256])
+@pytest.mark.parametrize("kind", ["one_cell", "rows_63", "rows_65", "flat", "long", "shuffled",
+                                  "star"])
+def test_tiles_sum_like_the_row_walk(cuda_device, kind, rows):
+    """Lumped diagonal (1 to 4 columns, Dirichlet rows) bit for bit; nodal gradient within
+    1e-12 of the largest one (the same sums; the compiler may contract a cell's cofactors
+    differently in two kernels), NaN at the same unused vertices."""
+    import torch
+    from dissolve_tp import _lib
+    from dissolve_tp.assembler import DeviceMesh
+    from dissolve_tp.device import ptr, stream_handle
+    xyz, cells = _mesh(kind)
+    dm = DeviceMesh(xyz, cells, tile_rows=0)
+    rng = np.random.default_rng(3)
+    V = dm.n_verts
+    u = torch.from_numpy(rng.uniform(-1.0, 1.0, V)).cuda()
+    mask = torch.from_numpy((rng.uniform(0, 1, V) < 0.2).astype(np.uint8)).cuda()
+    al = torch.from_numpy(rng.uniform(0, 1, (dm.n_cells, 4))).cuda()
+    grads, diags = [], []
+    for r in (0, rows):
+        dm.set_tiles(r)
+        g = torch.full((3 * V + 2,), -7.0, dtype=torch.float64, device="cuda")
+        _lib.call("tp_nodal_gradient", ctypes.byref(dm.tpm), None, ptr(u), ptr(g) + 8,
+                  stream_handle())
+        grads.append(g.cpu().numpy())
+        d = []
+        for S, ld in ((1, 1), (1, 2), (2, 2), (3, 3), (3, 4), (4, 4)):
+            d64 = torch.full((V * ld + 2,), -7.0, dtype=torch.float64, device="cuda")
+            d32 = torch.full((V * ld,), -7.0, dtype=torch.float32, device="cuda")
+            sh = (ctypes.c_double * 4)(0.5, 50.0, 0.0, 1e-3)
+            a = al[:, :ld].contiguous() if S != 2 else None
+            _lib.call("tp_lumped_diag", ctypes.byref(dm.tpm), S, ld, ptr(a), sh,
+                      ptr(mask) if ld > 1 else None, ptr(d64) + 8, ptr(d32), stream_handle())
+            d += [d64.cpu().numpy(), d32.cpu().numpy()]
+            assert d[-2][0] == -7.0 and d[-2][-1] == -7.0
+        diags.append(d)
+    for a, b in zip(*diags):
+        assert np.array_equal(a, b)
+    assert np.array_equal(np.isnan(grads[0]), np.isnan(grads[1]))
+    ref = np.nan_to_num(grads[0])
+    assert np.abs(np.nan_to_num(grads[1]) - ref).max() <= 1e-12 * np.abs(ref).max()
+    assert grads[1][0] == -7.0 and grads[1][-1] == -7.0
