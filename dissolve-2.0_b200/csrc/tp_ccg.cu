@@ -1698,7 +1698,12 @@ void fill(CcgArgs<VT>& a, const CcgClass* h, const CreateArgs& ca, int win_cap) 
   a.order = h->d_order;
   a.S = op->S;
   a.max_it = ca.max_it;
-  a.delta2 = ca.delta * ca.delta;
+  // FP32 recurrences drift: past a factor of some hundreds the true residual no longer
+  // follows theirs.  Ten steps of 274,625 rows and three species at rtol 1e-8 from the
+  // previous step: 3243 iterations with a refresh every factor 1000 (one step 480 instead of
+  // 230), 2703 at 300, 2697 at 100; a refresh costs about four iterations.
+  const double delta = sizeof(VT) == 4 ? std::max(ca.delta, 1.0 / 500.0) : ca.delta;
+  a.delta2 = delta * delta;
   a.slices = h->d_slices;
   a.loc_col = h->d_cols;
   a.push = h->d_push;

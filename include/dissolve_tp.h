@@ -534,8 +534,9 @@ TP_API int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block);
  * for systems of up to about 41k rows (one FP32 column), 25k (one FP64 column) or 16k (two
  * or three FP32 columns).  *window = 5: the same passes on every SM for larger systems, the
  * data exchanged with its pass number and no barrier per iteration (up to 1.3M rows for one
- * FP32 column, 450k for one FP64 column, 300k for three FP32 columns, while the windows fit
- * shared memory).  Engines 4 and 5 take no mass matrix, and are not chosen when the
+ * FP32 column, 450k for one FP64 column, 300k for three or four FP32 columns, while the
+ * windows fit shared memory).  Engines 4 and 5 take no mass matrix, refresh FP32 iterations
+ * at least every factor 500 whatever `delta` asks for, and are not chosen when the
  * environment names one of the others through a DISSOLVE_PCG_* variable or ctas_per_sm is
  * given; profiled runs use the grid engine of the handle.
  * *window = 0: the streaming engine (standard recurrences, columns and
