@@ -223,8 +223,10 @@ struct TcWait {
 };
 
 struct TcSmem {
-  __nv_bfloat16 A1[TC_R][TC_M * 16];     // features of the tile's 128-row parts, 4 KB each
-  __nv_bfloat16 A2[TC_R][4][TC_M * 16];  // their h1, one 4 KB block per K step
+  // of each 128-row part: h1, one 4 KB block per K step.  The features lie in the first
+  // block: layer 1 has read them before h1 is written, layer 2 has read h1 before the next
+  // tile's features (43 KB in all: no opt-in per launch).
+  __nv_bfloat16 A2[TC_R][4][TC_M * 16];
   __nv_bfloat16 W1[MLP_H * 16];    // 2 KB
   __nv_bfloat16 W2[4][MLP_H * 16]; // 8 KB
   alignas(16) float b1[MLP_H], b2[MLP_H], w3[MLP_H];
@@ -360,8 +362,7 @@ __global__ void __launch_bounds__(TC_M, TC_CTAS) k_mlp_predict(MlpFeat F, int64_
                                                       const float* __restrict__ P, float sigma,
                                                       double* __restrict__ x_out,
                                                       float* __restrict__ y_out, TcWait tw) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  TcSmem& sm = *reinterpret_cast<TcSmem*>(smem_raw);
+  __shared__ __align__(128) TcSmem sm;
   const int tid = threadIdx.x, warp = tid >> 5;
   // weights in the operand layout (BF16), biases and w3 (w3 rounded to BF16 as in training)
   // (every load of a thread in flight before its first conversion)
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(TC_M, TC_CTAS) k_mlp_predict(MlpFeat F, int64_
           const float hi = (in[q] && 2 * k + 1 < NFEAT) ? f[2 * k + 1] : 0.f;
           w[k] = pack_bf16(lo, hi);
         }
-        __nv_bfloat16* A = sm.A1[q];
+        __nv_bfloat16* A = sm.A2[q][0];
         *reinterpret_cast<uint4*>(A + tc_off(tid, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4*>(A + tc_off(tid, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
         base[q] = F.base == 1 ? 2.0 * cur[q].u - cur[q].up : (F.base == 0 ? cur[q].u : 0.0);
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(TC_M, TC_CTAS) k_mlp_predict(MlpFeat F, int64_
     if (tid == 0 && !tw.skip_issue) {
 #pragma unroll
       for (int q = 0; q < R; q++)
-        tc_mma(taddr + q * MLP_H, tc_desc(sm.A1[q]), tc_desc(sm.W1), 0);
+        tc_mma(taddr + q * MLP_H, tc_desc(sm.A2[q][0]), tc_desc(sm.W1), 0);
       tc_commit(&sm.bar);
     }
     r += step;
@@ -929,10 +930,7 @@ extern "C" int tp_mlp_predict(const tp_mlp_inputs* in, const float* params, floa
   if (tw.status) TP_CUDA_TRY(cudaMemsetAsync(tw.status, 0, sizeof(int32_t), st));
   const int64_t ntiles = (nrows + TC_ROWS - 1) / TC_ROWS;
   const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * TC_CTAS);
-  TP_CUDA_TRY(cudaFuncSetAttribute(k_mlp_predict, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(TcSmem)));
-  k_mlp_predict<<<grid, TC_M, sizeof(TcSmem), st>>>(make_feat(in), nrows, params, sigma, x_out,
-                                                    y_out, tw);
+  k_mlp_predict<<<grid, TC_M, 0, st>>>(make_feat(in), nrows, params, sigma, x_out, y_out, tw);
   TP_LAUNCH_CHECK();
   return TP_OK;
 }
