@@ -45,8 +45,9 @@ PARITY_STEPS = 3
 # relative residual of the oracle's Jacobi-PCG solves that stand in for exact solutions
 ORACLE_RTOL = 1e-12
 # measured with ncu on this workload (see profiles/); None until captured
-# (k_cgw: 2.627 GB over a 258-iteration launch; k_pcgp: 131.4 MB over a 334-iteration launch)
-DRAM_BYTES_PER_ITERATION = {"k_cgw": 10.2e6, "k_pcgp": 0.393e6}
+# (k_cgw: 2.627 GB over a 258-iteration launch; k_pcgp: 131.4 MB over a 334-iteration
+# launch; k_ccg: 126.1 MB over a 230-iteration launch)
+DRAM_BYTES_PER_ITERATION = {"k_cgw": 10.2e6, "k_pcgp": 0.393e6, "k_ccg": 0.548e6}
 WORKLOAD = ("3-species backward-Euler step, 64^3 Kuhn cube (1,572,864 P1 tets, 274,625 "
             "vertices), jitter 0.2h, De = D_s exp(0.3 xi), rtol 1e-8")
 
@@ -375,7 +376,7 @@ def roofline_solve(fast, flush, torch):
         # exchange engine: the same count
         bytes_it = nnz * 4 + 12 * nv * 16
         kernel = ("k_ccg<float,4,3,4,true> (persistent 3-column Jacobi-PCG on every SM, "
-                  "Chronopoulos-Gear form, vectors in registers, values in tensor memory, data "
+                  "Chronopoulos-Gear form, vectors and values in tensor memory, data "
                   "exchanged with its pass number, one cooperative launch per solve)")
         engine = "k_ccg"
     elif window:
@@ -399,7 +400,7 @@ def roofline_solve(fast, flush, torch):
     per_it = DRAM_BYTES_PER_ITERATION.get(engine)
     traffic = per_it * its if per_it else None
     peaks = _peaks()
-    # the driver-measured copy bandwidth of this pool's B200s, else the recipe's fallback
+    # the measured copy bandwidth, else the stated fallback
     hbm = float(peaks.get("hbm_gbs", 6650.0))
     peak_src = "of measured" if "hbm_gbs" in peaks else "of fallback: MEASURED_PEAKS.json absent"
     achieved = bytes_it * its / (solve_ms * 1e-3) / 1e9
@@ -657,7 +658,7 @@ def setup_times(m):
         out = {"device_mesh_s": round(t1 - t, 4), "tiles_s": round(t2 - t1, 4),
                "scatter_map_s": round(t3 - t2, 4),
                "includes": "H2D of coords and cells, geometry, incidence, pattern (two "
-                           "passes), slots; row tiles (host-built tables); scatter map built "
+                           "passes), slots; row tiles (built on the GPU); scatter map built "
                            "only on request"}
         del dm
     try:
