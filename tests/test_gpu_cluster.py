@@ -191,3 +191,40 @@ def test_exchange_solve_is_captured_in_a_graph(cuda_device):
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(sol.x, x) and sol.result()["iterations"] == ref["iterations"]
+
+
+@pytest.mark.parametrize("n,S,fp32", [(55, 3, True), (54, 4, True), (40, 1, False)])
+def test_exchange_engine_with_long_rows(cuda_device, monkeypatch, n, S, fp32):
+    """27-point rows: more entries than tensor memory holds per row, so the values are read
+    from shared memory or L2."""
+    import scipy.sparse as sp
+    import torch
+    from dissolve_tp.krylov import CsrOperator, PersistentCG
+    t = sp.diags([np.ones(n - 1), np.ones(n), np.ones(n - 1)], [-1, 0, 1])
+    A = (27.5 * sp.identity(n ** 3) - sp.kron(sp.kron(t, t), t)).tocsr()
+    A.sort_indices()
+    ld = {1: 1, 3: 4, 4: 4}[S]
+    V = n ** 3
+    K = torch.from_numpy(A.data).cuda()
+    rng = np.random.default_rng(n)
+    diag = torch.zeros((V, ld), dtype=torch.float64, device="cuda")
+    diag[:, :S] = torch.from_numpy(rng.uniform(0.5, 1.0, (V, S)))
+    op = CsrOperator(torch.from_numpy(A.indptr.astype(np.int32)).cuda(),
+                     torch.from_numpy(A.indices.astype(np.int32)).cuda(), K,
+                     K32=K.float() if fp32 else None, diag64=diag,
+                     diag32=diag.float() if fp32 else None, dscale=[1.0, 0.7, 2.6, 1.3][:S], S=S,
+                     ld=ld)
+    b = torch.zeros((V, ld), dtype=torch.float64, device="cuda")
+    b[:, :S] = torch.from_numpy(rng.uniform(-1.0, 1.0, (V, S)))
+    kw = dict(rtol=1e-11, max_it=4000, inner_fp32=fp32, delta=0.01)
+    one = PersistentCG(op, **kw)
+    monkeypatch.setenv("DISSOLVE_PCG_PIPE", "0")
+    grid = PersistentCG(op, **kw)
+    assert one.engine()["exchange"] and not grid.engine()["exchange"]
+    out = []
+    for sol in (one, grid):
+        sol.b.copy_(b)
+        sol.x.zero_()
+        _check(op, sol, sol.solve(), b, 1e-11)
+        out.append(sol.x.clone())
+    assert torch.linalg.norm(out[0] - out[1]) <= 1e-8 * torch.linalg.norm(out[1])
