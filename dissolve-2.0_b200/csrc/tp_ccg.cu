@@ -423,6 +423,10 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   __shared__ double s_red[CC_W][16];
   __shared__ __align__(8) uint64_t s_mb[3];  // partial sums (two buffers), halo
   __shared__ uint32_t s_taddr;
+  // Waits that ran out: set between two CTA barriers and read after the second.  A thread past
+  // that barrier may set it again in its next wait, so the two places that read it each ask for
+  // their own value, which all threads then read alike.
+  enum : int { GAVE_UP = 1, GAVE_UP_SUMS = 2 };  // the meeting or the halo; the sums
   __shared__ volatile int s_gave_up;
   // what warp 0 decided for the next pass (Ctl bits, refreshed columns) and its coefficients
   __shared__ int s_ctl, s_mask, s_run;
@@ -485,7 +489,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
           if ((int)(v - arrivals) >= 0) break;
           if (cc_time() - t0 > a.wait_limit_ns) {
-            s_gave_up = 1;
+            s_gave_up = GAVE_UP;
             break;
           }
         }
@@ -972,7 +976,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
 #pragma unroll
             for (int k = 0; k < 8; k++) {
               if (i0 + k * CC_T < part.nhalo) {
-                if (!poll_unit<TAG>(src[k], v[k], want, a.wait_limit_ns, &s_gave_up)) s_gave_up = 1;
+                if (!poll_unit<TAG>(src[k], v[k], want, a.wait_limit_ns, &s_gave_up)) s_gave_up = GAVE_UP;
                 const int i = nrows + i0 + k * CC_T;
                 const uint32_t w = (uint32_t)v[k].x;
                 memcpy(s_win + w_at(i, one), &w, 4);
@@ -999,7 +1003,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
 #pragma unroll
               for (int j = 0; j < UW; j++) {
                 if (!poll_unit<TAG>(src[k] + j, v[k][j], want, a.wait_limit_ns, &s_gave_up))
-                  s_gave_up = 1;
+                  s_gave_up = GAVE_UP;
                 if constexpr (sizeof(VT) == 8) {
                   uv[j] = __longlong_as_double((long long)v[k][j].x);
                 } else {
@@ -1016,7 +1020,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         }
         __syncthreads();
       } else {
-        if (!mb_wait(&s_mb[2], ph_halo, a.wait_limit_ns)) s_gave_up = 1;
+        if (!mb_wait(&s_mb[2], ph_halo, a.wait_limit_ns)) s_gave_up = GAVE_UP;
         ph_halo ^= 1u;
       }
 
@@ -1191,7 +1195,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         }
         __syncthreads();
         // a CTA that gave up sends no sums, so no other completes this pass either
-        if (s_gave_up) {
+        if (s_gave_up == GAVE_UP) {
           alive = false;
           break;
         }
@@ -1230,7 +1234,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
               for (int k = 0; k < 5; k++) {
                 if (b0 + 32 * k < (int)C) {
                   if (!poll_unit<0>(src + 32 * 16 * k, u[k], epoch, a.wait_limit_ns, &s_gave_up))
-                    s_gave_up = 1;
+                    s_gave_up = GAVE_UP_SUMS;
                   t2 += __longlong_as_double((long long)u[k].x);
                 }
               }
@@ -1243,7 +1247,8 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       // ---- warp 0: totals (lanes l and l + 16 sum half of the CTAs each), lane decisions
       if (warp == 0) {
         if constexpr (!GRID)
-          if (!mb_wait(&s_mb[buf], (ph_part >> buf) & 1u, a.wait_limit_ns)) s_gave_up = 1;
+          if (!mb_wait(&s_mb[buf], (ph_part >> buf) & 1u, a.wait_limit_ns))
+            s_gave_up = GAVE_UP_SUMS;
         double tot;
         if constexpr (GRID) {
           const double* pp = s_part + (lane & 15) + (lane >> 4) * 16 * 16;
@@ -1401,7 +1406,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       buf ^= 1u;
       epoch++;
       __syncthreads();
-      if (s_gave_up) {
+      if (s_gave_up == GAVE_UP_SUMS) {
         alive = false;
         break;
       }
