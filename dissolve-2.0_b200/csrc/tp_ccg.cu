@@ -22,9 +22,13 @@
 // are sent with st.async, whose bytes complete an mbarrier of the receiving CTA, so each of
 // the two exchanges costs one distributed-shared-memory latency.  A CTA may overwrite its
 // window because its neighbours send the next values only after they hold every CTA's
-// sums, which it sends after its product; the sums alternate between two buffers.  Waits
-// are bounded in time (tp_pcg_set_wait_limit); a CTA that gives up ends its solve with
-// TP_ERR_TIMEOUT and meets the others at the closing cluster barrier.
+// sums, which it sends after its product; the sums alternate between two buffers.  Before
+// an FP64 sweep the CTAs meet at an mbarrier where each arrives once at every other's.
+// Waits are bounded in time (tp_pcg_set_wait_limit).  A CTA that gives up ends its solve with
+// TP_ERR_TIMEOUT and takes part in no later exchange, so the others complete at most the
+// passes that it has sent its data for and then give up as well (or end converged).  The
+// closing cluster barrier is the only one after the start: a CTA leaves it, and frees its
+// shared memory, when none of the others starts another send.
 //
 // Layout.  The rows of a system are split into equal ranges of 32-row slices over the
 // cluster's CTAs.  r, p, s, xi and D^-1 of a row live in its thread's registers (thread =
@@ -60,6 +64,9 @@ namespace tp {
 
 constexpr int CC_T = 512, CC_W = CC_T / 32;
 constexpr unsigned long long CC_WAIT_NS = 2000000000ull;  // default bound of a wait: 2 s
+// how long a CTA whose wait ran out stays after the closing cluster barrier: no send starts
+// after it, and one in flight lands within about a microsecond
+constexpr unsigned long long CC_DRAIN_NS = 200000ull;
 constexpr int CC_SLOT_BITS = 14, CC_SRC_BITS = 13;  // push entry: rank | window slot | source row
 
 struct CcgPart {
@@ -139,6 +146,11 @@ __device__ __forceinline__ uint32_t cl_map(const void* smem, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(sa), "r"(rank));
   return r;
 }
+// one arrival at another CTA's mbarrier; publishes this CTA's writes before it to the cluster
+__device__ __forceinline__ void cl_mb_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mbar)
+               : "memory");
+}
 // asynchronous stores to another CTA's shared memory; the bytes complete its mbarrier
 __device__ __forceinline__ void cl_send(uint32_t dst, double v, uint32_t mbar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(
@@ -177,8 +189,9 @@ __device__ __forceinline__ void cl_send_row(uint32_t dst, const void* src, uint3
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
-__device__ __forceinline__ void mb_init(uint64_t* mb) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mb)) : "memory");
+__device__ __forceinline__ void mb_init(uint64_t* mb, uint32_t arrivals) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mb)), "r"(arrivals)
+               : "memory");
 }
 __device__ __forceinline__ void mb_expect(uint64_t* mb, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mb)),
@@ -421,7 +434,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   double* const s_part = reinterpret_cast<double*>(s_dyn);  // [2][rank][quantity * 4 + column]
   VT* const s_win = reinterpret_cast<VT*>(s_dyn + 2 * 16 * 16 * sizeof(double));
   __shared__ double s_red[CC_W][16];
-  __shared__ __align__(8) uint64_t s_mb[3];  // partial sums (two buffers), halo
+  __shared__ __align__(8) uint64_t s_mb[GRID ? 3 : 4];  // partial sums (two), halo, meeting
   __shared__ uint32_t s_taddr;
   // Waits that ran out: set between two CTA barriers and read after the second.  A thread past
   // that barrier may set it again in its next wait, so the two places that read it each ask for
@@ -474,10 +487,15 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   // GRID: 16-byte units of a published row, and where a unit keeps its pass number
   constexpr int UW = sizeof(VT) == 8 ? NC : (NC + 2) / 3;
   constexpr int TAG = sizeof(VT) == 8 ? 0 : 32;
-  uint32_t epoch = 1, arrivals = 0;
-  auto x_sync = [&]() {  // x written by every CTA of the system is visible to all
+  uint32_t epoch = 1, arrivals = 0, ph_x = 0;
+  // x written by every CTA of the system is visible to all.  A wait that runs out is acted on
+  // by this pass' check after the halo.
+  auto x_sync = [&]() {
     if constexpr (!GRID) {
-      cl_sync();
+      __syncthreads();
+      if (tid < (int)C) cl_mb_arrive(cl_map(&s_mb[3], (uint32_t)tid));
+      if (!mb_wait(&s_mb[3], ph_x, a.wait_limit_ns)) s_gave_up = GAVE_UP;
+      ph_x ^= 1u;
     } else {
       __syncthreads();
       if (tid == 0) {
@@ -517,7 +535,8 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
   if (warp == 0) cc_tm_alloc(&s_taddr);
   if (tid == 0) {
     s_gave_up = 0;
-    for (int k = 0; k < 3; k++) mb_init(&s_mb[k]);
+    for (int k = 0; k < 3; k++) mb_init(&s_mb[k], 1);
+    if constexpr (!GRID) mb_init(&s_mb[3], C + (a.wait_missing ? 1u : 0u));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1437,12 +1456,19 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
       }
     }
   }
-  // nothing is in flight towards a CTA that finished its solve; after a wait that ran out
-  // the others' sends may be: no CTA of a cluster leaves before all have given up
-  if constexpr (GRID)
+  // Nothing is in flight towards a CTA that finished its solve: it has received all that the
+  // others sent.  After a wait that ran out their last sends may be: the CTA stays until no
+  // other starts one (the barrier) and those in flight have landed.
+  if constexpr (GRID) {
     __syncthreads();
-  else
+  } else {
     cl_sync();
+    if (!alive) {
+      const unsigned long long t0 = cc_time();
+      while (cc_time() - t0 < CC_DRAIN_NS) {
+      }
+    }
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_taddr));
 }
