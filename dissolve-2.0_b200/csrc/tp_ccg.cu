@@ -732,8 +732,9 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     const bool is_col = lane < 4 && col < S;
     double st_alpha = 0.0, st_beta = 0.0, st_rmax2 = 0.0, st_tol2 = 0.0,
            st_bb = 0.0, st_rtrue = 0.0;
-    // 1 / rz and 1 / (rz alpha) of the last step (0: none yet)
-    double inv_rz = 0.0, inv_rza = 0.0;
+    // 1 / rz and 1 / alpha of the last step (0: none yet); their product would leave the FP64
+    // range for r.D^-1 r below 1e-154 or above 1e154
+    double inv_rz = 0.0, inv_al = 0.0;
     int st_act = 0, st_frozen = 0, st_status = TP_OK, st_iters = 0;
     unsigned tr_mask = (1u << S) - 1;  // columns refreshed by the next FP64 sweep
     bool refresh = true, first = true, fin = false;
@@ -1298,9 +1299,9 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           const double inv = 1.0 / gm;
           st_alpha = gm / den;
           inv_rz = inv;
-          inv_rza = den * inv * inv;
+          inv_al = den * inv;
         };
-        const double den0 = dl - gm * gm * inv_rza;
+        const double den0 = dl - (gm * inv_rz) * (gm * inv_al);
         // the common step: every running lane goes on, nothing to decide
         const bool runs = is_col && st_act && !st_frozen;
         const bool plain = rr > st_tol2 && !(rr < a.delta2 * st_rmax2) && rr < 1e300 &&
