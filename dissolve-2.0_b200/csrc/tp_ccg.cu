@@ -735,7 +735,9 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
     // 1 / rz and 1 / alpha of the last step (0: none yet); their product would leave the FP64
     // range for r.D^-1 r below 1e-154 or above 1e154
     double inv_rz = 0.0, inv_al = 0.0;
-    int st_act = 0, st_frozen = 0, st_status = TP_OK, st_iters = 0;
+    // STILL: at the tolerance, until a sweep confirms it
+    enum : int { DONE = 0, RUNS = 1, STILL = 2 };
+    int st_act = DONE, st_status = TP_OK, st_iters = 0;
     unsigned tr_mask = (1u << S) - 1;  // columns refreshed by the next FP64 sweep
     bool refresh = true, first = true, fin = false;
     int one = -1;  // ONE: the only column that still runs (the others stand still), or -1
@@ -1303,7 +1305,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         };
         const double den0 = dl - (gm * inv_rz) * (gm * inv_al);
         // the common step: every running lane goes on, nothing to decide
-        const bool runs = is_col && st_act && !st_frozen;
+        const bool runs = is_col && st_act == RUNS;
         const bool plain = rr > st_tol2 && !(rr < a.delta2 * st_rmax2) && rr < 1e300 &&
                            gm > 0.0 && gm < 1e300 && dl > 0.0 && den0 > 0.0 && den0 < 1e300;
         if (!refresh && it + 1 < a.max_it && !__any_sync(0xffffffffu, runs && !plain) &&
@@ -1326,24 +1328,24 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         if (!refresh) {
           it++;
           bool trig = false;
-          if (is_col && st_act && !st_frozen) {
+          if (runs) {
             if (!fine) {
               st_act = 0;
               st_status = TP_ERR_NONFINITE;
               st_iters = it;
             } else if (rr <= st_tol2) {
-              st_frozen = 1;
+              st_act = STILL;
             } else {
               trig = a.delta2 > 0.0 && rr < a.delta2 * st_rmax2;
             }
           }
-          const unsigned run = __ballot_sync(0xffffffffu, is_col && st_act && !st_frozen);
+          const unsigned run = __ballot_sync(0xffffffffu, is_col && st_act == RUNS);
           const unsigned act = __ballot_sync(0xffffffffu, is_col && st_act);
           if (__any_sync(0xffffffffu, trig) || (act && !run)) {
             ctl = CTL_REFRESH;
             tr_mask = act;
           } else {
-            coef = is_col && st_act && !st_frozen;
+            coef = is_col && st_act == RUNS;
           }
         } else if (first) {
           const double bb = __shfl_sync(0xffffffffu, tot, 12 + col);
@@ -1353,7 +1355,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
             st_tol2 = rt * rt * bb;
             st_rtrue = st_rmax2 = rr;
             const bool f = isfinite(rr) && isfinite(gm);
-            st_act = f && rr > st_tol2;
+            st_act = f && rr > st_tol2 ? RUNS : DONE;
             st_status = !f ? TP_ERR_NONFINITE : (st_act ? -1 : TP_OK);
             if (st_act && !isfinite(dl)) {
               st_act = 0;
@@ -1373,7 +1375,6 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
         } else {
           n_rel++;
           if (is_col && ((tr_mask >> col) & 1)) {
-            st_frozen = 0;
             st_rtrue = rr;
             if (!fine) {
               st_act = 0;
@@ -1394,10 +1395,13 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
             st_act = 0;
             st_status = TP_ERR_BREAKDOWN;
             st_iters = it;
-          } else if (den0 > 0.0) {
+          } else if (den0 > 0.0 && st_act == RUNS) {
             coefficients(den0, gm * inv_rz);
           } else {
-            coefficients(dl, 0.0);  // rounding: the direction restarts
+            // the direction restarts along u: rounding, or a column that stood still, whose p
+            // and q are overwritten meanwhile
+            coefficients(dl, 0.0);
+            st_act = RUNS;
           }
         }
         const unsigned act = __ballot_sync(0xffffffffu, is_col && st_act);
@@ -1409,7 +1413,7 @@ __global__ void __launch_bounds__(CC_T, 1) k_ccg(CcgArgs<VT> a) {
           ctl = bad ? CTL_REFRESH | CTL_FIN : CTL_EXIT;
           tr_mask = (1u << S) - 1;
         }
-        const bool go = is_col && st_act && !st_frozen;  // frozen lanes stand still
+        const bool go = is_col && st_act == RUNS;
         if (lane < 4) {
           s_al[lane] = go ? (VT)st_alpha : VT(0);
           s_be[lane] = go ? (VT)st_beta : VT(0);
