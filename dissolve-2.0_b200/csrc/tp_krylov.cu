@@ -1126,9 +1126,9 @@ extern "C" int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const 
     delete h;
     return TP_ERR_CUDA;
   }
-  // systems that fit one thread-block cluster each run there; the host-loop variant
-  // (use_graph_loop = 0) always is the graph engine
-  if (h->use_cond) {
+  // systems that fit one thread-block cluster each run there, unless the caller asks for the
+  // graph engine (use_graph_loop = 2, or 0 with its host loop)
+  if (cfg->use_graph_loop == 1) {
     rc = ccg_create(op, cfg->inner_fp32, CcgSource{}, cfg->max_it, delta, b, x, rtol,
                     false, st, &h->ccg);
     if (rc) {

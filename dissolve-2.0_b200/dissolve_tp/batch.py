@@ -3,10 +3,12 @@
 The meshes form one block-diagonal system (`mesh.concat_meshes`): one assembly launch
 over the union mesh (per-cell De and alpha carry each mesh's D and k), one right-hand-side
 launch, and one solve of every mesh as its own lane (`tp_cg_*` with n_systems = number
-of meshes: per-mesh dot products, convergence and iteration counts) run as a single CUDA
-graph with a device-side while loop.  Launch shape (threads per row, block, rows per
-reduction tile) comes from the project autotuner.  `MeshBatchPlain` is the comparison:
-the plain FP64 form, one mesh at a time.
+of meshes: per-mesh dot products, convergence and iteration counts).  Where every mesh fits
+one thread-block cluster each is solved by one (the cluster engine); otherwise, or when the
+caller gives a launch shape (`cg`: group, block, rows_per_tile), the solve is a single CUDA
+graph with a device-side while loop, whose launch shape comes from the project autotuner if
+the caller gives none.  `MeshBatchPlain` is the comparison: the plain FP64 form, one mesh at
+a time.
 
 The reference solves one field on one mesh per call (numerics/solvers.py:206-284); this
 batching is the multi-mesh form of that call.
@@ -78,16 +80,18 @@ class MeshBatch:
         self.op = CsrOperator(dm.indptr, dm.indices[: dm.nnz], self.K64, K32=self.K32,
                               n_systems=self.n_meshes, sys_row_ptr=vp)
         cg = dict(cg or {})
+        shaped = bool({"group", "block", "rows_per_tile"} & set(cg))
         self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32, **cg)
         if self.solver.cluster():
             self.cg_config = dict(engine="cluster", n_systems=self.n_meshes)
         else:
-            if autotune and not {"group", "block", "rows_per_tile"} & set(cg):
+            cg["engine"] = "graph"
+            if autotune and not shaped:
                 self.assemble_operator()
                 cg.update(tune_cg(self.op, inner_fp32=inner_fp32))
                 self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32,
                                        **cg)
-            self.cg_config = dict(cg, engine="graph", n_systems=self.n_meshes)
+            self.cg_config = dict(cg, n_systems=self.n_meshes)
         if asm_tiles is not None:
             self.cg_config["assembly_rows_per_tile"] = asm_tiles
         self.U = torch.zeros(dm.n_verts, dtype=torch.float64, device=dev)

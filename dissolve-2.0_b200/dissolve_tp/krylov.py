@@ -69,10 +69,22 @@ class CsrOperator:
 
 
 class CGSolver:
-    """Jacobi-PCG on every (system, column) lane, FP64 or FP32-inner + FP64 reliable updates."""
+    """Jacobi-PCG on every (system, column) lane, FP64 or FP32-inner + FP64 reliable updates.
+
+    engine: "auto" -- one thread-block cluster per system where every system fits one
+    (cluster() tells; FP32 inner iterations then refresh at least every factor 500, whatever
+    `delta` asks for), else the graph engine; "graph" -- always the graph engine.  Default:
+    "graph" when a launch shape (group, block, rows_per_tile: 4, 256, 256 unless given) is
+    given, since only that engine has one, else "auto".  use_graph_loop=False: the graph
+    engine with a host loop."""
 
     def __init__(self, op: CsrOperator, rtol=1e-8, max_it=1000, inner_fp32=False, delta=0.1,
-                 group=4, block=256, rows_per_tile=256, use_graph_loop=True):
+                 group=None, block=None, rows_per_tile=None, use_graph_loop=True, engine=None):
+        if engine is None:
+            shape = (group, block, rows_per_tile)
+            engine = "auto" if all(v is None for v in shape) else "graph"
+        if engine not in ("auto", "graph"):
+            raise ValueError(f"engine {engine!r} is not 'auto' or 'graph'")
         self.op = op
         dev = op.arrays["indptr"].device
         self.device = dev
@@ -85,10 +97,10 @@ class CGSolver:
         cfg.max_it = int(max_it)
         cfg.inner_fp32 = int(bool(inner_fp32))
         cfg.delta = float(delta)
-        cfg.group = int(group)
-        cfg.block = int(block)
-        cfg.rows_per_tile = int(rows_per_tile)
-        cfg.use_graph_loop = int(bool(use_graph_loop))
+        cfg.group = int(4 if group is None else group)
+        cfg.block = int(256 if block is None else block)
+        cfg.rows_per_tile = int(256 if rows_per_tile is None else rows_per_tile)
+        cfg.use_graph_loop = 0 if not use_graph_loop else (1 if engine == "auto" else 2)
         self.cfg = cfg
         nbytes = _lib.lib.tp_cg_workspace_bytes(ctypes.byref(op.struct), ctypes.byref(cfg))
         if nbytes == 0:

@@ -66,7 +66,8 @@ class PlainTransport:
                 self.solvers.append(PersistentCG(op, rtol=rtol, max_it=max_it,
                                                  sell=self.solvers[0].sell if s else None))
             else:
-                self.solvers.append(CGSolver(op, rtol=rtol, max_it=max_it, **cg))
+                self.solvers.append(CGSolver(op, rtol=rtol, max_it=max_it,
+                                             **dict(dict(engine="graph"), **cg)))
         self.engine = engine
         nv = self.asm[0].n_dofs
         self.U = [torch.zeros(nv, dtype=torch.float64, device=dev) for _ in range(self.S)]
@@ -172,7 +173,7 @@ class BatchedTransport:
                 cg.update(tune_cg(self.op, inner_fp32=inner_fp32))
             self.cg_config = dict(cg, engine="graph")
             self.solver = CGSolver(self.op, rtol=rtol, max_it=max_it, inner_fp32=inner_fp32,
-                                   delta=delta, **cg)
+                                   delta=delta, **self.cg_config)
         self.U = torch.zeros((n, self.ld), dtype=torch.float64, device=dev)
         self.U_prev = torch.zeros_like(self.U)
         # lumped mass per vertex (the cell-order sums of tp_lumped_diag with shift 1): the

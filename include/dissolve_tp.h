@@ -424,7 +424,9 @@ typedef struct tp_cg_config {
   int32_t group;         /* threads per CSR row: 1, 2, 4, 8 (autotuned)             */
   int32_t block;         /* threads per block: 128 or 256                           */
   int32_t rows_per_tile; /* rows per reduction tile (multiple of block/group)        */
-  int32_t use_graph_loop;/* 1: conditional-node while loop; 0: host loop            */
+  int32_t use_graph_loop;/* 1: conditional-node while loop, or the cluster engine where
+                            every system fits it (tp_cg_engine); 2: always the
+                            conditional-node loop; 0: host loop                     */
 } tp_cg_config;
 
 typedef struct tp_cg_result {
