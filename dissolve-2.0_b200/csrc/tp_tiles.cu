@@ -583,13 +583,11 @@ __global__ void __launch_bounds__(TB_T) k_tile_build(TileBuild b) {
       const int32_t v = b.indices[p];
       const int h1 = b.indptr[v + 1];
       int q = lower_bound(b.indices, b.indptr[v], h1, r);
-      if (q >= h1 || b.indices[q] != r) {
-        // an entry that no cell touches needs no partner
-        if (s_cnt[e]) tile_fail(b.err, TE_SYMMETRY, r, v);
-        q = p;
-      }
-      b.edge_pos[eb + e] = make_int2(p, q);
-      b.edge_rv[eb + e] = make_int2(r, v);
+      const bool pair = q < h1 && b.indices[q] == r;
+      // an entry that no cell touches needs no partner: its zero is written twice, to row r
+      if (!pair && s_cnt[e]) tile_fail(b.err, TE_SYMMETRY, r, v);
+      b.edge_pos[eb + e] = make_int2(p, pair ? q : p);
+      b.edge_rv[eb + e] = make_int2(r, pair ? v : r);
     }
   }
 }
