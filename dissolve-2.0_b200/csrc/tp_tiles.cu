@@ -385,6 +385,7 @@ struct TileBuild {
   const int32_t *start, *idx;
   const int32_t *vptr, *v2c, *indptr, *indices;
   const uint32_t* slots;
+  uint16_t* cnt;           // edge_cap counters per tile, or NULL: in shared memory
   int4* sizes;             // cells, diagonal terms, edges, edge terms of each tile
   TileError* err;
   // FILL: the tables
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(TB_T) k_tile_build(TileBuild b) {
   int32_t* s_tc = s_sort + b.cap;
   // ... then (FILL) the local index of every visit and the terms of every owned edge so far
   uint16_t* s_loc = reinterpret_cast<uint16_t*>(s_tc + (1 << TILE_LOC_BITS));
-  uint16_t* s_cnt = s_loc + b.cap;
+  uint16_t* s_cnt = b.cnt ? b.cnt + (int64_t)blockIdx.x * b.edge_cap : s_loc + b.cap;
   __shared__ int32_t s_row[TB_MAXR], s_vis[TB_MAXR + 1], s_edge[TB_MAXR + 1], s_dl[TB_MAXR];
   __shared__ int32_t s_scan[TB_T], s_kmax, s_kemax, s_bad;
   const int t = blockIdx.x, tid = threadIdx.x;
@@ -728,9 +729,17 @@ extern "C" int tp_tiles_create(const tp_mesh* m, int rows_per_tile, void* stream
   b.slots = m->v2c_slots;
   b.sizes = sizes;
   b.err = err;
-  b.edge_cap = std::min(h_most[1], 7 << TILE_LOC_BITS);  // six per cell, and some spare
+  b.edge_cap = h_most[1];
+  // the edges' counters: in shared memory up to six edges per cell and some spare (all that
+  // the pattern of a mesh asks for), else (a pattern with more entries) in device memory
+  const bool wide = b.edge_cap > (7 << TILE_LOC_BITS);
   const size_t smem = sizeof(int32_t) * ((size_t)b.cap + (1 << TILE_LOC_BITS)) +
-                      sizeof(uint16_t) * ((size_t)b.cap + (size_t)b.edge_cap);
+                      sizeof(uint16_t) * ((size_t)b.cap + (wide ? 0 : (size_t)b.edge_cap));
+  DeviceBuffer counters;
+  if (wide) {
+    TP_CUDA_TRY(cudaMalloc(&counters.p, sizeof(uint16_t) * (size_t)b.edge_cap * (size_t)nt));
+    b.cnt = reinterpret_cast<uint16_t*>(counters.p);
+  }
   std::vector<int4> h_sizes(nt);
   auto check = [&]() -> int {
     TileError e;

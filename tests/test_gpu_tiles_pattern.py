@@ -87,3 +87,9 @@ def test_entries_past_the_cells_are_zero(cuda_device, shape, upper, rows):
     for x, y in zip(want, got):
         assert np.array_equal(x, y)
     assert np.all(got[0][~p.touched] == 0.0) and np.all(got[1][~p.touched] == 0.0)
+
+
+def test_more_entries_than_a_meshs_tile_can_own(cuda_device):
+    """125 entries past each diagonal: tiles of 256 rows own 32,000, more than the six edges
+    of each of 4,095 cells."""
+    test_entries_past_the_cells_are_zero(cuda_device, (2, 2, 150), 125, 256)
