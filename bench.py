@@ -414,8 +414,9 @@ def roofline_solve(fast, flush, torch):
                     "state from the previous-step guess; the operator and vectors stay on "
                     "chip (tensor memory, shared memory) and in the 126 MB L2 between "
                     "iterations, so the solve is bound by its exchanges and on-chip "
-                    "latencies, not by DRAM; traffic = ncu DRAM bytes per iteration x "
-                    "iterations of this launch"}
+                    "latencies, not by DRAM, and frac (algorithmic bytes / time / peak) may "
+                    "pass 1; traffic = ncu DRAM bytes per iteration x iterations of this "
+                    "launch"}
 
 
 def guess_ablation(fast, u0, args, flush, torch):
@@ -518,6 +519,8 @@ def kernel_table(m, coef, u0, flush):
         # consistent mass: cell vertices (16 B) and |detJ| (8 B) per cell, u and b per vertex
         "rhs_3col_consistent": (lambda: _lib.call("tp_assemble_rhs", tpm, 3, 4, ptr(U), None, 50.0,
                                                   0, 0, None, None, ptr(b), st), n * 24 + V * 64),
+        # connectivity, De and coordinates (the kernel reads 64-byte geometry records in the
+        # coordinates' place: 56 B a cell more), x and y per vertex
         "matfree_3col_fp64": (lambda: _lib.call("tp_matfree_apply", tpm, 3, 4, 0, ptr(De), None,
                                                 ds, sh, 50.0, 0, 0, ptr(x64), ptr(y64), st),
                               n * 40 + V * 72),
@@ -574,9 +577,9 @@ def matrix_free_solve(dm, De, U, flush, torch):
     its = max(int(res["iterations"]), 1)
     return {"ms": round(ms, 3), "iterations": its, "us_per_iteration": round(ms * 1e3 / its, 2),
             "converged": bool(res["converged"]),
-            "note": "FP64, 3 lanes, previous-step guess; every product recomputes the "
-                    "gradients (tp_matfree_apply), iterations in batches of 8 between host "
-                    "checks"}
+            "note": "FP64, 3 lanes, previous-step guess; every product is a matrix-free apply "
+                    "from the geometry records (tp_matfree_apply), iterations in batches of "
+                    "8 between host checks"}
 
 
 def reference_kernel_baseline(dm, De, alpha, ours64, flush, hbm):

@@ -4,8 +4,8 @@ Same names and call signatures: libceed_available, make_ceed, extract_ceed_mesh_
 compute_geometric_factors, build_elem_restriction, build_simplex_basis and
 CeedDiffusionMassOp(ceed, mesh_data, De_vals, inv_dt, num_comp=1) with .apply(u, out)
 and .update_coeffs(De_vals, inv_dt).  libCEED is replaced by the fused matrix-free kernel
-tp_matfree_apply, which recomputes each cell's P1 gradients from the vertex coordinates
-in FP64 (no stored quadrature-point geometry).
+tp_matfree_apply, which reads each cell's FP64 geometry record (J^-1 J^-T and |det J|; no
+stored quadrature-point geometry).
 
 Semantics.  The operator is a(u, v) = (inv_dt u, v) + (De grad u, grad v) with De the
 mean of the vertex values on each cell (ceed_operators.py:330-339) and the consistent P1

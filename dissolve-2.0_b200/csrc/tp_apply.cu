@@ -22,10 +22,13 @@
 // Bound by latency and by the L1's handling of gathers and atomics, not by memory: the
 // records cost 56 bytes per cell more than the coordinates but half the gathers, no
 // division and 20 registers; the vertices of a thread's next cell are loaded a turn ahead,
-// so a turn waits for memory once; the grid is what is resident (4 blocks an SM: 44.0 us a
-// call, 3 or twice as many blocks than resident 46 to 48).  1,572,864 cells, one FP64
-// column: 46.7 us from coordinates, 39.1 from records, 31.0 with the loads ahead and the
-// runs summed by shuffles instead of through shared memory.
+// so a turn waits for memory once; the grid is what is resident (calls of 1,572,864 cells
+// with the L2 flushed before each: 44.0 us with 4 blocks an SM, 46 to 48 with 3, 5 or twice
+// as many blocks as resident).  The kernel alone on those cells, one FP64 column: 46.7 us
+// from coordinates, 39.1 from records, 31.0 with the loads ahead and the runs summed by
+// shuffles instead of through shared memory.  Clear and kernel together, from coordinates and
+// in this form, us: 3,072 cells 3.5 and 3.1, 82,944 5.2 and 4.7, 384,000 11.8 and 8.5; three
+// FP64 columns 4.7 and 4.4, 7.8 and 7.4, 18.6 and 18.8.
 #include "tp_ops.cuh"
 
 namespace tp {
@@ -782,8 +785,7 @@ extern "C" int tp_guess_project(const tp_csr_op* op, const double* diag, const u
 
 // ================================================================= matrix-free Krylov solve
 // Jacobi-preconditioned CG whose product is the matrix-free apply above (k_matfree): the
-// operator is never assembled, every product recomputes the P1 gradients from the
-// coordinates.  This is the solve of the reference's MatShell branch
+// operator is never assembled.  This is the solve of the reference's MatShell branch
 // (numerics/solvers.py:172-203, 375-404: PETSc KSP around CeedDiffusionMassOp) on the GPU.
 // FP64, S columns of LD; Dirichlet rows are identity rows (x = b there, the
 // preconditioner zero), as in the CSR engines.  Reductions are one FP64 partial per block

@@ -771,8 +771,10 @@ __global__ void k_rhs_bc(int64_t n_bc, const int32_t* __restrict__ bc, int64_t n
 // Sums over a row's cells of N values that depend on the cell alone.  A tile's cells compute
 // theirs once into shared memory (N planes, the last slot zero for the padding terms); then
 // a thread per row and value adds the row's terms in ascending cell order, 8 at a time: the
-// sums of the row walks, bit for bit, with each cell's arithmetic and loads done by about 1.7
-// tiles instead of by all 4 of its rows, which walked them one cell's latency at a time.
+// sums of the row walks, with each cell's arithmetic and loads done by about 1.7 tiles
+// instead of by all 4 of its rows, which walked them one cell's latency at a time.  The lumped
+// diagonal is theirs bit for bit; the gradient from coordinates within rounding, since the
+// compiler may contract a cell's cofactors differently in the two kernels.
 // out(row, n, sum) is called by whole warps, N consecutive lanes per row (row < 0: none).
 // Bound by the L1's gathers of the cells' data and the shared-memory reads of the terms;
 // BLOCKS per SM as measured (more until the registers spill; several cells of a thread side

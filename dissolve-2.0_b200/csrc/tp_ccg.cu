@@ -3,17 +3,17 @@
 // A solve of a few thousand to a few ten thousand rows is bound by the latency of its two
 // synchronisations per iteration, not by its arithmetic: over the whole chip each costs a
 // grid barrier and an L2 round trip for the partial sums.  A system that fits 8 or 16 SMs
-// is solved here by one cluster: barriers are the hardware's cluster barrier, partial sums
-// and the halo of the shared vector travel through distributed shared memory, and several
-// systems run side by side, one per cluster, the largest first.
+// is solved here by one cluster: partial sums and the halo of the shared vector travel
+// through distributed shared memory, and several systems run side by side, one per cluster,
+// the largest first.
 //
 // Chronopoulos-Gear form, the recurrences of k_cgw (tp_pcg.cu):
 //
 //   loop  p = u + beta p, s = w + beta s, xi += alpha p, r -= alpha s, u = D^-1 r
 //         u into the CTA's window and pushed into the windows that hold it as halo
-//                                                            | cluster barrier
-//         w = A u;  r.u, r.r, w.u to every CTA of the cluster | cluster barrier
-//         totals, lane decisions, alpha, beta (every warp, same bits)
+//                                                            | the halo's bytes have come
+//         w = A u;  r.u, r.r, w.u to every CTA of the cluster | the sums' bytes have come
+//         totals, lane decisions, alpha, beta (one warp of every CTA, same bits)
 //   when a lane asks (FP32 inner: its recurrence residual fell by delta; both: it reached
 //   the tolerance and no lane still runs): x += xi, r = b - A x in FP64, and the loop goes
 //   on from there.  Convergence is declared on that FP64 residual only.

@@ -192,7 +192,9 @@ class SellPattern:
 class PersistentCG:
     """The same Jacobi-PCG as CGSolver for one system, as one cooperative kernel per solve
     (tp_pcg_*).  The inner operator is read in SELL-32 order: call refresh_values() after the
-    CSR values change (it scatters them)."""
+    CSR values change (it scatters them).  delta: FP32 iterations are refreshed in FP64 when
+    a residual has fallen by it; the cluster and exchange engines do so at least every factor
+    500 (delta 0.002) and the pipelined engine every factor 1000, whatever it asks for."""
 
     def __init__(self, op: CsrOperator, rtol=1e-8, max_it=1000, inner_fp32=False, delta=0.01,
                  sell: SellPattern | None = None, ctas_per_sm: int = 0):
@@ -247,7 +249,9 @@ class PersistentCG:
                 self.sell.scatter(a["M64"], out64=self.sM)
 
     def profile_run(self) -> dict:
-        """One solve with per-CTA phase clocks; mean and max over CTAs in microseconds."""
+        """One solve with per-CTA phase clocks; mean and max over CTAs in microseconds.  It
+        runs and times the handle's grid engine, also where solves run the cluster or
+        exchange engine."""
         g, _ = self.grid()
         prof = torch.zeros(g * 8, dtype=torch.int64, device=self.device)
         call("tp_pcg_set_profile", self._h, ptr(prof))
@@ -262,13 +266,15 @@ class PersistentCG:
                 "min_us": dict(zip(names, p.min(0).round(1).tolist()))}
 
     def set_wait_limit(self, limit_s: float = 0.0, missing_arrivals: int = 0):
-        """Bound of every grid-barrier wait of the next solves (0: the 2 s default).
-        missing_arrivals > 0 is for tests of the failure path: every barrier then waits for
-        that many CTAs that do not exist, so the solve ends with TP_ERR_TIMEOUT after
-        limit_s; set it back to 0 for normal solves (the handle stays usable)."""
+        """Bound of every wait of the next solves (0: the 2 s default).  missing_arrivals > 0
+        is for tests of the failure path: every wait then expects something that never comes
+        (a barrier that many CTAs, an exchange that many bytes or passes more), so the solve
+        ends with TP_ERR_TIMEOUT after limit_s; set it back to 0 for normal solves (the handle
+        stays usable)."""
         call("tp_pcg_set_wait_limit", self._h, int(round(limit_s * 1e9)), int(missing_arrivals))
 
     def grid(self):
+        """Grid and block of the handle's grid engine (the shape of its profile)."""
         g, b = ctypes.c_int(0), ctypes.c_int(0)
         call("tp_pcg_grid", self._h, ctypes.byref(g), ctypes.byref(b))
         return int(g.value), int(b.value)
@@ -276,8 +282,8 @@ class PersistentCG:
     def engine(self) -> dict:
         """Engine of the handle: shared-memory window (Chronopoulos-Gear; `tmem`: with the
         recurrence vectors in tensor memory; `pipelined`: the one-barrier pipelined form,
-        vectors in tensor memory; `cluster`: one thread-block cluster; `exchange`: every SM, data exchanged
-        with its pass number and no barrier per iteration) or streaming."""
+        vectors in tensor memory; `cluster`: one thread-block cluster; `exchange`: every SM,
+        data exchanged with its pass number and no barrier per iteration) or streaming."""
         w, sm = ctypes.c_int(0), ctypes.c_size_t(0)
         call("tp_pcg_engine", self._h, ctypes.byref(w), ctypes.byref(sm))
         return {"window": bool(w.value), "tmem": w.value in (2, 3), "pipelined": w.value == 3,
@@ -319,8 +325,8 @@ class PersistentCG:
 class MatrixFreeCG:
     """Jacobi-PCG whose product is the matrix-free apply (tp_mfcg_solve): the operator of
     tp_matfree_apply -- per column s, sum_e [dscale_s De_e K_e + (inv_dt + alpha_e +
-    shift_s) M_e] -- is never assembled; every product recomputes the P1 gradients from the
-    coordinates.  The solve of the reference's MatShell branch (numerics/solvers.py:172-203,
+    shift_s) M_e] -- is never assembled; every product reads the cells' geometry records.
+    The solve of the reference's MatShell branch (numerics/solvers.py:172-203,
     375-404) on the GPU.  b, x: (n_verts, ld) FP64 device arrays; x is the initial guess
     and receives the solution."""
 

@@ -358,8 +358,8 @@ typedef struct tp_csr_op {
 
 /* [sync] Matrix-free Jacobi-PCG (numerics/solvers.py:172-203, 375-404: the reference's
  * PETSc KSP around the CeedDiffusionMassOp MatShell): solves A x = b for S interleaved
- * columns, A the operator of tp_matfree_apply (same arguments), every product recomputing
- * the P1 gradients from coords4; nothing is assembled.  FP64.  bc_mask (or NULL): those
+ * columns, A the operator of tp_matfree_apply (same arguments), every product one
+ * tp_matfree_apply (geometry records, or coords4 where geo is NULL); nothing is assembled.  FP64.  bc_mask (or NULL): those
  * rows are identity rows (x = b there).  rtol (host, S values): stops each lane when its
  * recurrence residual ||r||_2 <= rtol ||b||_2, then confirms it on ||b - A x||_2 (reported
  * per lane in res).  x: initial guess in, solution out.  workspace: 256-byte aligned,
@@ -452,7 +452,8 @@ TP_API int tp_cg_create(const tp_csr_op* op, const tp_cg_config* cfg, const doub
 /* Engine the handle runs (chosen at create).  *cluster = 1: every system is solved by one
  * thread-block cluster (all systems fit one: about 70k rows for one FP32 column, 49k for
  * one FP64 column, 24k for 4 FP32 columns; no mass matrix; use_graph_loop = 1), which
- * ignores group, block and rows_per_tile; 0: the graph engine. */
+ * ignores group, block and rows_per_tile and refreshes FP32 iterations at least every factor
+ * 500 whatever `delta` asks for; 0: the graph engine. */
 TP_API int tp_cg_engine(tp_cg_handle* h, int* cluster);
 
 /* enqueue one solve (recomputes the Jacobi diagonal from the current values) */
@@ -535,7 +536,7 @@ TP_API int tp_pcg_grid(tp_pcg_handle* h, int* grid, int* block);
  * `delta` asks for.  *window = 4: the Chronopoulos-Gear form in one thread-block cluster,
  * for systems of up to about 41k rows (one FP32 column), 25k (one FP64 column) or 16k (two
  * or three FP32 columns).  *window = 5: the same passes on every SM for larger systems, the
- * data exchanged with its pass number and no barrier per iteration (up to 1.3M rows for one
+ * data exchanged with its pass number and no barrier per iteration (up to 680k rows for one
  * FP32 column, 450k for one FP64 column, 300k for three or four FP32 columns, while the
  * windows fit shared memory).  Engines 4 and 5 take no mass matrix, refresh FP32 iterations
  * at least every factor 500 whatever `delta` asks for, and are not chosen when the
