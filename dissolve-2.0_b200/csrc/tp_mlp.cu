@@ -350,8 +350,10 @@ __device__ __forceinline__ uint32_t bias_relu_bf16(uint32_t z0, uint32_t z1, uin
 // x_out[v, s] = B[v, s] + sigma * y(v, s)  (or y_out[r] = y when x_out is NULL).
 // Every thread gathers all features of its row (no divergent per-feature branches).
 //
-// Bound by the epilogues' instruction issue and shared-memory reads, not by the tensor
-// cores or memory.  So: bias, BF16 rounding and maximum on packed pairs; the biases and w3
+// Bound by the serial chain of a CTA (features, MMA, wait, epilogue, MMA, wait, epilogue): with
+// three CTAs an SM half of the issue slots stay empty and the tensor pipe runs a quarter of the
+// time; DRAM is at 18 %.  What shortens the chain are fewer instructions and shared-memory
+// reads in it.  So: bias, BF16 rounding and maximum on packed pairs; the biases and w3
 // (16 bytes a read, the same for every lane) read once for two rows; the weights read with
 // every load in flight; one barrier less per tile.  823,875 rows: 50 us with one row per
 // thread and scalar epilogues, 45.7 with packed ones, 36.7 with the weights' loads batched,
